@@ -82,6 +82,9 @@ def _space(bench, dtype):
                     out.append({"JACOBI_HW_WARPS": hw, "JACOBI_CHUNK": ch, "JACOBI_BANDS": 0,
                                 "JACOBI_TMA": 2})
     elif bench == "heat_3d":
+        if f64:  # the limb form, which has one setting; the rows select the integer form
+            for ch in (0, 1, 2, 3, 4, 6, 8, 10, 12, 16):
+                out.append({"HEAT_ROWS": 0, "HEAT_HW_ROWS": -1, "HEAT_CHUNK": ch})
         for rows in (1, 2, 4):
             tj = 8 * rows
             for hw in (sorted({0, tj // 8, tj // 4, 5 * tj // 16, 3 * tj // 8, 7 * tj // 16})

@@ -42,6 +42,8 @@ extern int64_t g_cfg_heat_tb;
 extern int64_t g_cfg_heat_stages;
 extern int64_t g_cfg_heat_mad_rows;
 
+int32_t heat3d_limb_run(double* a, double* b, int64_t n0, int64_t n1, int64_t n2, int32_t tsteps,
+                        cudaStream_t st);
 int32_t heat3d_tb2_run(float* a, float* b, int64_t n0, int64_t n1, int64_t n2, int32_t tsteps,
                        cudaStream_t st, int32_t (*single_pairs)(float*, float*, int64_t, int64_t,
                                                                 int64_t, int32_t, cudaStream_t));
@@ -390,6 +392,16 @@ int32_t launch_ldg(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tstep
 template <typename T, bool FX>
 int32_t run_single(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tsteps, cudaStream_t st) {
   if (tsteps <= 1 || n0 < 3 || n1 < 3 || n2 < 3) return NPBGB_OK;
+  // Exact binary64 additions run in binary32 limbs (heat_limb.cu) unless a knob
+  // of the integer form is set: faster at every size measured (ms at TSTEPS=21,
+  // limbs / integers: 25^3 0.15 / 0.22, 70^3 0.28 / 0.55, 120^3 0.61 / 0.78, 256^3 3.7 / 4.9).
+  if constexpr (FX) {
+    if (g_cfg_heat_tma && g_cfg_heat_rows == 0 && g_cfg_heat_hw_rows < 0 && g_cfg_heat_mad_rows == 0 &&
+        g_cfg_f64_cvt == 0) {
+      const int32_t r = heat3d_limb_run(a, b, n0, n1, n2, tsteps, st);
+      if (r != NPBGB_ERR_STATE) return r;
+    }
+  }
   if (g_cfg_heat_tma) {
     // Tuned on GB300 (256^3): binary32 is memory-latency bound and wants more
     // rows per thread; binary64 (integer-pipe bound) wants one.
