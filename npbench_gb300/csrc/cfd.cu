@@ -9,8 +9,9 @@
 //   p        nit pressure iterations (:24-38), each from the previous iterate;
 //   u, v     the momentum updates (:53-74) from copies un, vn and the new p.
 // All of them run here in ONE cooperative persistent launch for the whole
-// time loop.  The interior rows are cut into bands, one band per CTA.  A band
-// starts sweep s once both neighbouring bands have finished sweep s-1 (their
+// time loop.  The interior rows are cut into bands, one band per CTA.  Grids
+// whose bands fit in shared memory take cfd_mail (below); the others cfd_bands,
+// which works in global memory.  There a band starts sweep s once both neighbouring bands have finished sweep s-1 (their
 // counters, published with release semantics after their stores and read
 // with acquire semantics), so no grid-wide barrier is needed.  Two buffers
 // per field (ping-pong) make that wait enough for write-after-read as well: the
@@ -39,12 +40,14 @@
 // thread), and publishes a continue/stop word the other bands wait on.  A cap
 // on the step count keeps a non-converging input from running forever.
 //
-// Every operator is one correctly rounded IEEE operation (divisions are
-// __ddiv_rn, never multiplication by a reciprocal), in the reference's order,
+// Every operator is one correctly rounded IEEE operation (divisions by the
+// loop's constants in cfd_mail take four operations to the same bits,
+// divisor.cuh), in the reference's order,
 // with the scalars it forms in Python computed the same way (its dx**2 is the
 // C library's pow), so results are bit-identical to NumPy's.  Grids with
 // fewer than 3 rows or columns have no interior and take a one-CTA kernel that
 // executes the boundary statements literally.
+#include "divisor.cuh"
 #include "npbgb_common.cuh"
 
 #include <math.h>
@@ -61,6 +64,7 @@ constexpr int kCThreads = 256;
 constexpr uint64_t kCfdLimitNs = 2000000000ull;
 
 struct CfdConsts {
+  Divisor by_two_dx, by_two_dy, by_dx, by_dy, by_pD;  // (mailbox form)
   double two_dx, two_dy, inv_dt, dx2, dy2, pD, pC, k1u, k1v, k2, k3;
   double dt, dx, dy, rho, nu;
 };
@@ -92,6 +96,9 @@ struct CfdArgs {
   double* val;                 // global home of val when it exceeds kSumSmem
   uint32_t* ctl;               // steps allowed to start; kStop bit: finished
   int64_t* steps_out;          // step count (negative: stopped by max_steps)
+  // mailbox form only
+  ulonglong2* p_mail;          // [band][side][slot][nx]
+  ulonglong2* uv_mail;         // [band][side][slot][u, v][nx]
 };
 
 constexpr uint32_t kStop = 0x80000000u;
@@ -208,7 +215,7 @@ __device__ double numpy_sum_cta(const CfdArgs& a, const double* u) {
   __shared__ double sval[kSumSmem];
   double* val = 2 * a.nleaves - 1 <= kSumSmem ? sval : a.val;
   const int q = threadIdx.x & 7, grp = threadIdx.x >> 3;
-  for (int32_t base = 0; base < a.nleaves; base += kCThreads / 8) {
+  for (int32_t base = 0; base < a.nleaves; base += int32_t(blockDim.x) / 8) {
     const int32_t l = base + grp;
     const bool live = l < a.nleaves;
     const int32_t n = live ? a.leaf_len[l] : 0;
@@ -235,7 +242,7 @@ __device__ double numpy_sum_cta(const CfdArgs& a, const double* u) {
   }
   __syncthreads();
   for (int32_t h = 0; h < a.nlevels; ++h) {
-    for (int32_t k = a.lvl[h] + threadIdx.x; k < a.lvl[h + 1]; k += kCThreads)
+    for (int32_t k = a.lvl[h] + threadIdx.x; k < a.lvl[h + 1]; k += int32_t(blockDim.x))
       val[a.node_out[k]] = add_rn(val[a.node_l[k]], val[a.node_r[k]]);
     __syncthreads();
   }
@@ -251,7 +258,7 @@ __device__ bool channel_decide(const CfdArgs& a, uint32_t s, int32_t n, const do
   // One thread per band counter, so the polls overlap.
   int r = 1;
   const uint64_t t0 = globaltimer();
-  for (int bb = threadIdx.x; bb < a.nbands && r; bb += kCThreads)
+  for (int bb = threadIdx.x; bb < a.nbands && r; bb += int(blockDim.x))
     while (ld_acquire(a.done + bb) < s) {
       if (globaltimer() - t0 > kCfdLimitNs) {
         atomicOr(&g_cfd_error, 1u);
@@ -409,6 +416,392 @@ cfd_bands(CfdArgs a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// The mailbox form, for grids whose bands fit in shared memory
+// ---------------------------------------------------------------------------
+// The time loop is a chain of dependent sweeps, so its speed is the hand-off
+// between neighbouring bands plus one row's arithmetic.  cfd_bands spends
+// 2.5 us a sweep at 101 x 101: stores, a release counter, an acquire poll, then
+// reads of the neighbour's row through L2.  Here
+//   * a band's rows of u, v, p and pC*b stay in shared memory;
+//   * an edge value travels as one 16-byte element {value, sweep number}, written
+//     and polled with single-copy-atomic 128-bit accesses by the two threads
+//     that own the column, so one trip through L2 carries data and signal, and
+//     nothing waits for a whole row (0.71 us a sweep with no arithmetic);
+//   * the half of a point that needs no neighbouring band, (p_e + p_w)*dy^2, is
+//     evaluated while the mail is under way;
+//   * divisions are by the loop's constants (div_by).
+// The binary64 pipe takes 77 clocks for an operation of four warps, so the eight
+// that follow the mail are 0.3 us of the 1.15 us a sweep takes now; the rest is the
+// trip through L2 and the CTA barrier.  Measured (ms, before / now): cavity 101^2,
+// 700 steps of 50 iterations 88.1 / 41.9; 201^2, 100 of 20 9.12 / 4.92; 61^2, 25 of
+// 5 0.53 / 0.28; channel 121^2, 10 iterations 42.5 / 18.8; 201^2, 20 130 / 51.
+//
+// Elements alternate between two slots.  A thread writes sweep s over s-2 of its
+// column after it has received sweep s-1 of the same column from the same
+// neighbour, which that neighbour's thread sent after it had received s-2.
+//
+// Channel flow: an extra CTA decides.  It sums u once every band has stored its
+// rows of step n, while the bands already run b and the pressure iterations of
+// step n+1 on a copy; they wait for the verdict before they change u and v, and
+// fall back to the copy of p when it is to stop.
+constexpr int kMailFields = 7;  // p twice, pC*b, u twice, v twice
+
+__device__ __forceinline__ void post(ulonglong2* at, double v, uint64_t tag) {
+  asm volatile("{\n.reg .b128 q;\nmov.b128 q, {%1, %2};\nst.relaxed.gpu.global.b128 [%0], q;\n}" ::"l"(at),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ void peek(const ulonglong2* at, uint64_t& v, uint64_t& tag) {
+  asm volatile("{\n.reg .b128 q;\nld.relaxed.gpu.global.b128 q, [%2];\nmov.b128 {%0, %1}, q;\n}"
+               : "=l"(v), "=l"(tag)
+               : "l"(at)
+               : "memory");
+}
+// Waits for the N elements at[k] (those with need[k]) to carry `tag`; false
+// after the time limit.
+template <int N>
+__device__ __forceinline__ bool collect(const ulonglong2* const (&at)[N], bool (&need)[N], uint64_t tag,
+                                        double (&v)[N]) {
+  uint64_t t0 = 0;
+  for (uint32_t n = 1;; ++n) {
+    bool missing = false;
+    uint64_t x[N], t[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (need[k]) peek(at[k], x[k], t[k]);
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (need[k]) {
+        if (t[k] == tag) {
+          v[k] = __longlong_as_double(static_cast<long long>(x[k]));
+          need[k] = false;
+        } else {
+          missing = true;
+        }
+      }
+    if (!missing) return true;
+    if ((n & 255u) == 0) {
+      const uint64_t now = globaltimer();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kCfdLimitNs) {
+        atomicOr(&g_cfd_error, 1u);
+        return false;
+      }
+    }
+  }
+}
+
+// Channel flow's verdicts.  ctl counts the steps that may change u and v.
+__device__ void channel_judge(const CfdArgs& a) {
+  double s_prev = numpy_sum_cta(a, a.u[0]);
+  if (threadIdx.x == 0) st_release(a.ctl, 1u);
+  for (uint32_t n = 1;; ++n) {
+    int r = 1;
+    const uint64_t t0 = globaltimer();
+    for (int bb = threadIdx.x; bb < a.nbands && r; bb += int(blockDim.x))
+      while (ld_acquire(a.done + bb) < n)
+        if (globaltimer() - t0 > kCfdLimitNs) {
+          atomicOr(&g_cfd_error, 1u);
+          r = 0;
+          break;
+        }
+    if (!__syncthreads_and(r)) return;
+    const double su = numpy_sum_cta(a, a.u[0]);
+    bool stop = false;
+    if (threadIdx.x == 0) {
+      const double udiff = ddiv(sub_rn(su, s_prev), su);
+      const bool more = udiff > 0.001;
+      stop = !more || int64_t(n) >= a.max_steps;
+      if (stop) *a.steps_out = more ? -int64_t(n) : int64_t(n);
+      __threadfence();
+      st_release(a.ctl, stop ? kStop : n + 1u);
+    }
+    s_prev = su;
+    if (__syncthreads_or(stop)) return;
+  }
+}
+
+template <bool CH, int CPT>
+__global__ void __launch_bounds__(kCThreads)
+cfd_mail(CfdArgs a) {
+  if (CH && int(blockIdx.x) == a.nbands) {
+    channel_judge(a);
+    return;
+  }
+  extern __shared__ double field[];
+  const int b = blockIdx.x, nb = a.nbands, T = blockDim.x;
+  const int nx = int(a.nx), ny = int(a.ny);
+  const int r0 = 1 + b * a.rows;
+  const int R = (r0 + a.rows < ny - 1 ? r0 + a.rows : ny - 1) - r0;
+  const int size = a.rows * nx;
+  auto P = [&](int which) { return field + which * size; };
+  double* const CB = field + 2 * size;
+  auto U = [&](int which) { return field + (3 + which) * size; };
+  auto V = [&](int which) { return field + (5 + which) * size; };
+  double* const PS = field + kMailFields * size;  // channel flow
+  const CfdConsts& k = a.k;
+  const bool lowest = b == 0, highest = b == nb - 1;
+
+  // This thread's columns; act: columns it evaluates.
+  int col[CPT], oe[CPT], ow[CPT];
+  bool act[CPT];
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {
+    const int j = int(threadIdx.x) + c * T;
+    col[c] = j;
+    act[c] = CH ? j < nx : (j >= 1 && j < nx - 1);
+    oe[c] = CH ? (j + 1 == nx ? 0 : j + 1) : j + 1;
+    ow[c] = CH ? (j == 0 ? nx - 1 : j - 1) : j - 1;
+  }
+  for (int o = threadIdx.x; o < R * nx; o += T) {
+    const int64_t g = int64_t(r0) * nx + o;
+    P(0)[o] = L(a.p[0] + g);
+    U(0)[o] = L(a.u[0] + g);
+    V(0)[o] = L(a.v[0] + g);
+  }
+  // Halo rows (above: row r0-1, below: row r0+R) of this thread's columns.
+  double pa[CPT], pb[CPT], ua[CPT], ub[CPT], va[CPT], vb[CPT];
+#pragma unroll
+  for (int c = 0; c < CPT; ++c)
+    if (act[c]) {
+      const int64_t ga = int64_t(r0 - 1) * nx + col[c], gb = int64_t(r0 + R) * nx + col[c];
+      pa[c] = L(a.p[0] + ga);
+      pb[c] = L(a.p[0] + gb);
+      ua[c] = L(a.u[0] + ga);
+      ub[c] = L(a.u[0] + gb);
+      va[c] = L(a.v[0] + ga);
+      vb[c] = L(a.v[0] + gb);
+    }
+  auto p_box = [&](int band, int side, uint64_t tag) {
+    return a.p_mail + (int64_t(band * 2 + side) * 2 + int64_t(tag & 1)) * nx;
+  };
+  auto uv_box = [&](int band, int side, uint64_t tag, int which) {
+    return a.uv_mail + ((int64_t(band * 2 + side) * 2 + int64_t(tag & 1)) * 2 + which) * nx;
+  };
+  __syncthreads();
+
+  int cu = 0, pc = 0;
+  uint64_t sweeps = 0, halo = 0;  // pressure iterations done; those pa and pb belong to
+  bool ok = true;
+  // p's halo rows after the newest iteration.
+  auto p_halo = [&]() {
+    if (halo == sweeps) return;
+    halo = sweeps;
+    const double* p = P(pc);
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+      if (!act[c]) continue;
+      const ulonglong2* at[2] = {p_box(lowest ? b : b - 1, 1, sweeps) + col[c],
+                                 p_box(highest ? b : b + 1, 0, sweeps) + col[c]};
+      bool need[2] = {!lowest, !highest};
+      double v[2];
+      v[0] = p[col[c]];                                     // row 0 = row 1
+      v[1] = CH ? p[(R - 1) * nx + col[c]] : 0.0;           // row ny-1
+      if (ok) ok = collect<2>(at, need, sweeps, v);
+      pa[c] = v[0];
+      pb[c] = v[1];
+    }
+  };
+
+  const int steps = CH ? 0x7fffffff : a.nt;
+  bool stopped = false;
+  for (int n = 0; n < steps; ++n) {
+    const double* u = U(cu);
+    const double* v = V(cu);
+    if (n > 0) {
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        if (!act[c]) continue;
+        const int up = lowest ? b : b - 1, dn = highest ? b : b + 1;
+        const ulonglong2* at[4] = {uv_box(up, 1, n, 0) + col[c], uv_box(up, 1, n, 1) + col[c],
+                                   uv_box(dn, 0, n, 0) + col[c], uv_box(dn, 0, n, 1) + col[c]};
+        bool need[4] = {!lowest, !lowest, !highest, !highest};
+        double x[4] = {0.0, 0.0, CH ? 0.0 : 1.0, 0.0};  // the walls
+        if (ok) ok = collect<4>(at, need, uint64_t(n), x);
+        ua[c] = x[0];
+        va[c] = x[1];
+        ub[c] = x[2];
+        vb[c] = x[3];
+      }
+      if (__syncthreads_or(!ok)) return;
+    }
+    // pC * b (build_up_b)
+    for (int i = 0; i < R; ++i) {
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        if (!act[c]) continue;
+        const int o = i * nx + col[c];
+        const double un = i > 0 ? u[o - nx] : ua[c], us = i + 1 < R ? u[o + nx] : ub[c];
+        const double vn = i > 0 ? v[o - nx] : va[c], vs = i + 1 < R ? v[o + nx] : vb[c];
+        const double x1 = div_by(sub_rn(u[i * nx + oe[c]], u[i * nx + ow[c]]), k.by_two_dx);
+        const double x2 = div_by(sub_rn(vs, vn), k.by_two_dy);
+        double r = mul_rn(k.inv_dt, add_rn(x1, x2));
+        r = sub_rn(r, mul_rn(x1, x1));
+        double z = div_by(sub_rn(us, un), k.by_two_dy);
+        z = mul_rn(z, sub_rn(v[i * nx + oe[c]], v[i * nx + ow[c]]));
+        z = div_by(z, k.by_two_dx);
+        r = sub_rn(r, mul_rn(2.0, z));
+        r = sub_rn(r, mul_rn(x2, x2));
+        CB[o] = mul_rn(k.pC, mul_rn(k.rho, r));
+        if (CH) PS[o] = P(pc)[o];
+      }
+    }
+    // Pressure iterations
+    for (int q = 0; q < a.nit; ++q) {
+      const double* x = P(pc);
+      double* y = P(pc ^ 1);
+      const uint64_t tag = sweeps + 1;
+      auto ew = [&](int i, int c) {
+        return mul_rn(add_rn(x[i * nx + oe[c]], x[i * nx + ow[c]]), k.dy2);
+      };
+      auto finish = [&](int i, int c, double s, double north, double south) {
+        s = add_rn(s, mul_rn(add_rn(south, north), k.dx2));
+        const int o = i * nx + col[c];
+        const double val = sub_rn(div_by(s, k.by_pD), CB[o]);
+        y[o] = val;
+        if (!CH) {  // columns 0 and nx-1 equal their neighbours
+          if (col[c] == 1) y[o - 1] = val;
+          if (col[c] == nx - 2) y[o + 1] = val;
+        }
+        return val;
+      };
+      double first[CPT], last[CPT];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c)
+        if (act[c]) {
+          first[c] = ew(0, c);
+          if (R > 1) last[c] = ew(R - 1, c);
+        }
+      p_halo();
+#pragma unroll
+      for (int c = 0; c < CPT; ++c)
+        if (act[c]) {
+          const double val = finish(0, c, first[c], pa[c], R > 1 ? x[nx + col[c]] : pb[c]);
+          if (!lowest) post(p_box(b, 0, tag) + col[c], val, tag);
+          if (R == 1 && !highest) post(p_box(b, 1, tag) + col[c], val, tag);
+        }
+      if (R > 1) {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+          if (act[c]) {
+            const double val = finish(R - 1, c, last[c], x[(R - 2) * nx + col[c]], pb[c]);
+            if (!highest) post(p_box(b, 1, tag) + col[c], val, tag);
+          }
+        for (int i = 1; i < R - 1; ++i) {
+#pragma unroll
+          for (int c = 0; c < CPT; ++c)
+            if (act[c]) finish(i, c, ew(i, c), x[(i - 1) * nx + col[c]], x[(i + 1) * nx + col[c]]);
+        }
+      }
+      sweeps = tag;
+      pc ^= 1;
+      if (__syncthreads_or(!ok)) return;
+    }
+    // u and v
+    p_halo();
+    if (CH) {
+      int go = 1;  // 1: run, 0: stop, -1: gave up
+      if (threadIdx.x == 0) {
+        const uint64_t t0 = globaltimer();
+        for (;;) {
+          const uint32_t w = ld_acquire(a.ctl);
+          if (w & kStop) { go = 0; break; }
+          if (w >= uint32_t(n) + 1u) break;
+          if (globaltimer() - t0 > kCfdLimitNs) {
+            atomicOr(&g_cfd_error, 1u);
+            go = -1;
+            break;
+          }
+        }
+      }
+      if (__syncthreads_or(!ok || go < 0)) return;
+      if (__syncthreads_or(go == 0)) {
+        stopped = true;
+        break;
+      }
+    } else if (__syncthreads_or(!ok)) {
+      return;
+    }
+    {
+      const double* p = P(pc);
+      double* uo = U(cu ^ 1);
+      double* vo = V(cu ^ 1);
+      auto momentum = [&](const double* f, int i, int c, double fn, double fs, double cx, double cy,
+                          double pdiff, double k1) {
+        const int o = i * nx + col[c];
+        const double fc = f[o], fe = f[i * nx + oe[c]], fw = f[i * nx + ow[c]];
+        const double x = mul_rn(cx, sub_rn(fc, fw));
+        const double y = mul_rn(cy, sub_rn(fc, fn));
+        const double out = sub_rn(sub_rn(sub_rn(fc, x), y), mul_rn(k1, pdiff));
+        const double two_f = mul_rn(2.0, fc);
+        const double d1 = mul_rn(k.k2, add_rn(sub_rn(fe, two_f), fw));
+        const double d2 = mul_rn(k.k3, add_rn(sub_rn(fs, two_f), fn));
+        return add_rn(out, mul_rn(k.nu, add_rn(d1, d2)));
+      };
+      const uint64_t tag = uint64_t(n) + 1;
+      for (int i = 0; i < R; ++i) {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          if (!act[c]) continue;
+          const int o = i * nx + col[c];
+          const double cx = div_by(mul_rn(u[o], k.dt), k.by_dx);
+          const double cy = div_by(mul_rn(v[o], k.dt), k.by_dy);
+          const double un = i > 0 ? u[o - nx] : ua[c], us = i + 1 < R ? u[o + nx] : ub[c];
+          const double vn = i > 0 ? v[o - nx] : va[c], vs = i + 1 < R ? v[o + nx] : vb[c];
+          const double pn = i > 0 ? p[o - nx] : pa[c], ps = i + 1 < R ? p[o + nx] : pb[c];
+          double nu_ = momentum(u, i, c, un, us, cx, cy, sub_rn(p[i * nx + oe[c]], p[i * nx + ow[c]]), k.k1u);
+          if (CH) nu_ = add_rn(nu_, a.fdt);
+          const double nv_ = momentum(v, i, c, vn, vs, cx, cy, sub_rn(ps, pn), k.k1v);
+          uo[o] = nu_;
+          vo[o] = nv_;
+          if (i == 0 && !lowest) {
+            post(uv_box(b, 0, tag, 0) + col[c], nu_, tag);
+            post(uv_box(b, 0, tag, 1) + col[c], nv_, tag);
+          }
+          if (i == R - 1 && !highest) {
+            post(uv_box(b, 1, tag, 0) + col[c], nu_, tag);
+            post(uv_box(b, 1, tag, 1) + col[c], nv_, tag);
+          }
+          if (CH) {
+            __stcg(a.u[0] + int64_t(r0 + i) * nx + col[c], nu_);
+            if (n == 0 && i == 0 && lowest) __stcg(a.u[0] + col[c], 0.0);
+            if (n == 0 && i == R - 1 && highest) __stcg(a.u[0] + int64_t(ny - 1) * nx + col[c], 0.0);
+          }
+        }
+        if (!CH && threadIdx.x == 0) {  // the side walls
+          uo[i * nx] = uo[i * nx + nx - 1] = 0.0;
+          vo[i * nx] = vo[i * nx + nx - 1] = 0.0;
+        }
+      }
+    }
+    cu ^= 1;
+    __syncthreads();
+    if (CH && threadIdx.x == 0) red_release_add(a.done + b, 1u);
+  }
+  // Results.  The pressure is untouched without iterations.
+  const double* p = CH && stopped ? PS : P(pc);
+  for (int o = threadIdx.x; o < R * nx; o += T) {
+    const int64_t g = int64_t(r0) * nx + o;
+    a.u[0][g] = U(cu)[o];
+    a.v[0][g] = V(cu)[o];
+    if (a.nit > 0) a.p[0][g] = p[o];
+  }
+  for (int j = threadIdx.x; j < nx; j += T) {
+    const int64_t g = int64_t(ny - 1) * nx + j;
+    if (lowest) {
+      a.u[0][j] = 0.0;
+      a.v[0][j] = 0.0;
+      if (a.nit > 0) a.p[0][j] = p[j];
+    }
+    if (highest) {
+      a.u[0][g] = CH ? 0.0 : 1.0;
+      a.v[0][g] = 0.0;
+      if (a.nit > 0) a.p[0][g] = CH ? p[(R - 1) * nx + j] : 0.0;
+    }
+  }
+}
+
 // Grids with fewer than 3 rows or columns: no interior point exists, so b and
 // the interior updates are empty and only the boundary statements act; one CTA
 // runs them in the reference's order.
@@ -477,6 +870,11 @@ CfdConsts make_consts(double dt, double dx, double dy, double rho, double nu) {
   k.k1v = dt / t;
   k.k2 = dt / dx2;
   k.k3 = dt / dy2;
+  k.by_two_dx = divisor(k.two_dx);
+  k.by_two_dy = divisor(k.two_dy);
+  k.by_dx = divisor(dx);
+  k.by_dy = divisor(dy);
+  k.by_pD = divisor(k.pD);
   k.dt = dt;
   k.dx = dx;
   k.dy = dy;
@@ -508,10 +906,72 @@ constexpr int64_t kAlign = 256;
 int64_t round_up(int64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 }  // namespace
 
-extern "C" int64_t npbgb_cavity_flow_workspace_bytes(int64_t ny, int64_t nx) {
-  if (ny <= 0 || nx <= 0) return 0;
+namespace {
+// The mailbox form of a grid: one band per CTA (channel flow keeps an SM for the
+// CTA that judges), a thread per one, two or four columns; bands must fit in
+// shared memory.  Larger grids take cfd_bands.
+struct MailPlan {
+  bool fits = false;
+  int64_t nb = 0, rows = 0, p_bytes = 0, uv_bytes = 0;
+  int threads = 0, per_thread = 0;
+  size_t smem = 0;
+};
+constexpr size_t kMailSmem = 190 * 1024;  // next to the judge's static 33 KB
+
+MailPlan mail_plan(int64_t ny, int64_t nx, bool channel) {
+  MailPlan m;
+  if (ny < 3 || nx < (channel ? 2 : 3) || nx > 4 * npbgb::kCThreads) return m;
+  const int64_t sms = npbgb::sm_count() - (channel ? 1 : 0);
+  m.rows = npbgb::cdiv(ny - 2, sms);
+  m.nb = npbgb::cdiv(ny - 2, m.rows);
+  m.per_thread = nx <= npbgb::kCThreads ? 1 : nx <= 2 * npbgb::kCThreads ? 2 : 4;
+  m.threads = nx <= npbgb::kCThreads ? int(npbgb::cdiv(nx, 32) * 32) : npbgb::kCThreads;
+  if (channel && m.threads < 128) m.threads = 128;  // the judge sums with them
+  m.smem = size_t(npbgb::kMailFields + (channel ? 1 : 0)) * size_t(m.rows * nx) * sizeof(double);
+  m.p_bytes = round_up(m.nb * 4 * nx * int64_t(sizeof(ulonglong2)));
+  m.uv_bytes = 2 * m.p_bytes;
+  m.fits = m.smem <= kMailSmem;
+  return m;
+}
+
+cudaError_t launch_cooperative(const void* kernel, unsigned ctas, unsigned threads, size_t smem,
+                               cudaStream_t st, npbgb::CfdArgs& a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3{ctas, 1, 1};
+  cfg.blockDim = dim3{threads, 1, 1};
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  void* args[] = {&a};
+  return npbgb::counted(cudaLaunchKernelExC(&cfg, kernel, args));
+}
+
+// The kernel for a plan, ready to launch cooperatively; nullptr with `e` set on failure.
+template <bool CH>
+const void* mail_kernel(const MailPlan& m, cudaError_t& e) {
+  using namespace npbgb;
+  const void* k = m.per_thread == 1   ? reinterpret_cast<const void*>(cfd_mail<CH, 1>)
+                  : m.per_thread == 2 ? reinterpret_cast<const void*>(cfd_mail<CH, 2>)
+                                      : reinterpret_cast<const void*>(cfd_mail<CH, 4>);
+  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kMailSmem));
+  return e == cudaSuccess ? k : nullptr;
+}
+
+int64_t cavity_bands_bytes(int64_t ny, int64_t nx) {
   const int64_t field = round_up(ny * nx * int64_t(sizeof(double)));
   return 4 * field + round_up(cfd_bands(ny) * int64_t(sizeof(uint32_t)));
+}
+}  // namespace
+
+extern "C" int64_t npbgb_cavity_flow_workspace_bytes(int64_t ny, int64_t nx) {
+  if (ny <= 0 || nx <= 0) return 0;
+  const MailPlan m = mail_plan(ny, nx, false);
+  const int64_t bands = cavity_bands_bytes(ny, nx), mail = m.p_bytes + m.uv_bytes;
+  return m.fits && mail > bands ? mail : bands;
 }
 
 extern "C" int32_t npbgb_cavity_flow(void* u, void* v, void* p, int64_t ny, int64_t nx, int32_t nt,
@@ -539,7 +999,7 @@ extern "C" int32_t npbgb_cavity_flow(void* u, void* v, void* p, int64_t ny, int6
   }
   const int64_t need = npbgb_cavity_flow_workspace_bytes(ny, nx);
   void* ws = workspace;
-  if (ws != nullptr && workspace_bytes < need)
+  if (ws != nullptr && workspace_bytes < cavity_bands_bytes(ny, nx))
     return set_error(NPBGB_ERR_ARG, "cavity_flow: workspace of %lld bytes, %lld needed",
                      (long long)workspace_bytes, (long long)need);
   if (ws == nullptr) {
@@ -570,19 +1030,21 @@ extern "C" int32_t npbgb_cavity_flow(void* u, void* v, void* p, int64_t ny, int6
   a.rows = int32_t(cdiv(ny - 2, nb));
   a.k = make_consts(dt, dx, dy, rho, nu);
   int32_t status = NPBGB_OK;
-  cudaError_t e = cudaMemsetAsync(a.done, 0, size_t(nb) * sizeof(uint32_t), st);
-  if (e == cudaSuccess) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3{unsigned(nb), 1, 1};
-    cfg.blockDim = dim3{unsigned(kCThreads), 1, 1};
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    void* args[] = {&a};
-    e = counted(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(cfd_bands<false>), args));
+  cudaError_t e = cudaSuccess;
+  const MailPlan m = mail_plan(ny, nx, false);
+  if (m.fits && (workspace == nullptr || workspace_bytes >= m.p_bytes + m.uv_bytes)) {
+    a.p_mail = reinterpret_cast<ulonglong2*>(w);
+    a.uv_mail = reinterpret_cast<ulonglong2*>(w + m.p_bytes);
+    a.nbands = int32_t(m.nb);
+    a.rows = int32_t(m.rows);
+    e = cudaMemsetAsync(w, 0, size_t(m.p_bytes + m.uv_bytes), st);
+    const void* kern = e == cudaSuccess ? mail_kernel<false>(m, e) : nullptr;
+    if (kern) e = launch_cooperative(kern, unsigned(m.nb), unsigned(m.threads), m.smem, st, a);
+  } else {
+    e = cudaMemsetAsync(a.done, 0, size_t(nb) * sizeof(uint32_t), st);
+    if (e == cudaSuccess)
+      e = launch_cooperative(reinterpret_cast<const void*>(cfd_bands<false>), unsigned(nb),
+                             unsigned(kCThreads), 0, st, a);
   }
   if (e != cudaSuccess) status = cuda_status(e, "cavity_flow: cooperative launch");
   if (workspace == nullptr) cudaFreeAsync(ws, st);
@@ -651,7 +1113,7 @@ SumPlan sum_plan(int64_t n) {
 
 struct ChannelLayout {
   int64_t field, nb, nleaves, nnodes, nlevels, off_done, off_leaf_off, off_leaf_len, off_node_l,
-      off_node_r, off_node_out, off_lvl, off_val, off_ctl, off_steps, total;
+      off_node_r, off_node_out, off_lvl, off_val, off_ctl, off_steps, bands_total, off_mail, total;
 };
 
 ChannelLayout channel_layout(int64_t ny, int64_t nx, const SumPlan& p) {
@@ -672,7 +1134,12 @@ ChannelLayout channel_layout(int64_t ny, int64_t nx, const SumPlan& p) {
   l.off_val = o;       o += round_up((l.nleaves + l.nnodes) * 8);
   l.off_ctl = o;       o += kAlign;
   l.off_steps = o;     o += kAlign;
-  l.total = o;
+  l.bands_total = o;   // what the band form needs
+  // The mailboxes take the place of the band form's second buffers where they fit.
+  const MailPlan m = mail_plan(ny, nx, true);
+  const int64_t mail = m.fits ? m.p_bytes + m.uv_bytes : 0;
+  l.off_mail = mail <= 4 * l.field ? 0 : o;
+  l.total = l.off_mail > 0 ? o + mail : o;
   return l;
 }
 }  // namespace
@@ -702,7 +1169,7 @@ extern "C" int32_t npbgb_channel_flow(void* u, void* v, void* p, int64_t ny, int
   const SumPlan plan = sum_plan(ny * nx);
   const ChannelLayout l = channel_layout(ny, nx, plan);
   void* ws = workspace;
-  if (ws != nullptr && workspace_bytes < l.total)
+  if (ws != nullptr && workspace_bytes < l.bands_total)
     return set_error(NPBGB_ERR_ARG, "channel_flow: workspace of %lld bytes, %lld needed",
                      (long long)workspace_bytes, (long long)l.total);
   if (ws == nullptr) {
@@ -764,18 +1231,18 @@ extern "C" int32_t npbgb_channel_flow(void* u, void* v, void* p, int64_t ny, int
     if (ny < 3) {
       channel_small<<<1, kCThreads, 0, st>>>(a);
       e = counted(cudaGetLastError());
+    } else if (const MailPlan m = mail_plan(ny, nx, true);
+               m.fits && (workspace == nullptr || workspace_bytes >= l.total)) {
+      a.p_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail);
+      a.uv_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail + m.p_bytes);
+      a.nbands = int32_t(m.nb);
+      a.rows = int32_t(m.rows);
+      e = cudaMemsetAsync(w + l.off_mail, 0, size_t(m.p_bytes + m.uv_bytes), st);
+      const void* kern = e == cudaSuccess ? mail_kernel<true>(m, e) : nullptr;
+      if (kern) e = launch_cooperative(kern, unsigned(m.nb + 1), unsigned(m.threads), m.smem, st, a);
     } else {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3{unsigned(l.nb), 1, 1};
-      cfg.blockDim = dim3{unsigned(kCThreads), 1, 1};
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeCooperative;
-      attr[0].val.cooperative = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      void* args[] = {&a};
-      e = counted(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(cfd_bands<true>), args));
+      e = launch_cooperative(reinterpret_cast<const void*>(cfd_bands<true>), unsigned(l.nb),
+                             unsigned(kCThreads), 0, st, a);
     }
   }
   if (e == cudaSuccess && steps != nullptr) {
