@@ -104,14 +104,13 @@ extern "C" {
                                          planes per CTA; 0 (default) = automatic */
 #define NPBGB_CFG_JACOBI_BANDS 18     /* jacobi2d: the whole time loop in one launch with
                                          bands of rows resident in shared memory.
-                                         2: whenever the bands fit; 0 (default) or 1:
-                                         chained launches (measured faster over mixed
-                                         shapes and under concurrent streams; the
-                                         autotuner picks 2 per shape class where it
-                                         wins).  Results are identical either way. */
-#define NPBGB_CFG_JACOBI_BANDS_WARPS 19 /* warps per CTA of that kernel: 8, 16 or 32;
-                                           0 (default): one 32-column strip per warp,
-                                           8 to 32 warps */
+                                         1 (default): where they measured faster
+                                         (binary32 that fits, small binary64 grids);
+                                         2: whenever the bands fit; 0: chained
+                                         launches.  Results are identical either way. */
+#define NPBGB_CFG_JACOBI_BANDS_WARPS 19 /* 8, 16, 32 or 0 (default); kept for callers
+                                           that set it: the bands' threads follow from
+                                           the grid's width */
 #define NPBGB_CFG_HEAT_STAGES 20      /* heat3d binary32 TMA kernel: depth of the
                                          shared-memory plane ring, 4, 6 or 8;
                                          0 (default) = automatic */
@@ -245,9 +244,10 @@ NPBGB_API int32_t npbgb_probe_pipe(int32_t op, int64_t iters, int32_t ctas, void
  *   dst = 0.2 * ((((c + w) + e) + s) + n)
  * Boundary rows and columns are never written.  On return A holds the newest
  * field and B the previous one, as in the reference.  tsteps <= 1 is a no-op.
- * One chained launch per half-sweep; with NPBGB_CFG_JACOBI_BANDS = 2, grids
- * whose bands of rows fit in shared memory run the whole loop in one
- * cooperative launch (its exchange rows come from a stream-ordered pool). */
+ * Grids whose bands of rows fit in shared memory run the whole loop in one
+ * cooperative launch where that measured faster (NPBGB_CFG_JACOBI_BANDS; its
+ * exchange rows come from a stream-ordered pool), any other in one chained launch
+ * per half-sweep. */
 NPBGB_API int32_t npbgb_jacobi2d(void* A, void* B, int64_t ny, int64_t nx, int32_t tsteps,
                        int32_t dtype, void* stream);
 

@@ -28,8 +28,8 @@ int64_t g_cfg_jacobi1d_ctas = 0;   // 0: default
 int64_t g_cfg_jacobi1d_depth = 0;  // 0: default
 int64_t g_cfg_heat_tb = 0;         // binary32 Heat-3D half-sweeps per launch (0: by size)
 int64_t g_cfg_heat_tb_chunk = 0;   // 0: automatic
-int64_t g_cfg_jacobi_bands = 0;    // 0, 1: chained launches; 2: bands whenever they fit
-int64_t g_cfg_jacobi_bands_warps = 0;  // 0: by the grid's width
+int64_t g_cfg_jacobi_bands = 1;    // 0: chained launches; 1: bands where they measured faster; 2: whenever they fit
+int64_t g_cfg_jacobi_bands_warps = 0;  // kept for callers that set it
 int64_t g_cfg_heat_stages = 0;         // 0: automatic (8)
 int64_t g_cfg_heat_mad_rows = 0;
 int64_t g_cfg_queue_whole_cells = 65536;

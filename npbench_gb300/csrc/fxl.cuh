@@ -57,6 +57,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cmath>
 #include <cstring>
 
 #include "fx64.cuh"
@@ -138,17 +139,15 @@ NPBGB_FX_FN P2 add_rz(P2 a, P2 b) {
   });
 #endif
 }
-// a * b + c with one rounding.  Differences are written as multiply-adds by
-// minus one: the packed add negates no operand, so a packed subtraction costs
-// two more logic instructions (measured: 27 a point of Heat-3D).  The host products here are by powers of two or
-// exact, so that a plain multiply and add round once as well.
+// a * b + c with one rounding.  Differences are written as multiply-adds by minus
+// one, which take a constant operand the kernels hold anyway.
 NPBGB_FX_FN P2 fma(P2 a, P2 b, P2 c) {
 #if defined(__CUDA_ARCH__)
   P2 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
   return r;
 #else
-  return each(a, b, c, [](float x, float y, float z) { return x * y + z; });
+  return each(a, b, c, [](float x, float y, float z) { return std::fma(x, y, z); });
 #endif
 }
 NPBGB_FX_FN P2 fma_rz(P2 a, P2 b, P2 c) {
@@ -158,7 +157,7 @@ NPBGB_FX_FN P2 fma_rz(P2 a, P2 b, P2 c) {
   return r;
 #else
   return each(a, b, c, [](float x, float y, float z) {
-    return toward_zero(x, y, z, [](float p, float q, float s) { return p * q + s; });
+    return toward_zero(x, y, z, [](float p, float q, float s) { return std::fma(p, q, s); });
   });
 #endif
 }
@@ -184,7 +183,8 @@ constexpr uint32_t kNaN = 0x7fffffffu;
 // being rebuilt (two moves) at every use.
 struct Consts {
   P2 h_base, m_base, l_base, one, minus_one, l_to_m, h_scale, minus_two, eight;
-  uint32_t implicit;
+  P2 fifth, minus_five, m_to_l, t_to_l, z_scale, third;  // (fifth_of)
+  uint32_t implicit, half_bit;
 };
 NPBGB_FX_FN uint32_t opaque(uint32_t v) {
 #if defined(__CUDA_ARCH__)
@@ -207,6 +207,13 @@ NPBGB_FX_FN Consts consts() {
   k.h_scale = opaque_both(0x83800000u);  // -2^-120
   k.minus_two = opaque_both(0xc0000000u);
   k.eight = opaque_both(0x41000000u);
+  k.fifth = opaque_both(0x3e4cccccu);       // just below 1/5
+  k.minus_five = opaque_both(0xc0a00000u);
+  k.m_to_l = opaque_both(0x4e000000u);      // 2^29
+  k.t_to_l = opaque_both(0x33000000u);      // 2^-25
+  k.z_scale = opaque_both(0x49cccccdu);     // 2^23 / 5
+  k.third = opaque_both(0x3eaaaa80u);       // (1 - 2^-18) / 3
+  k.half_bit = opaque(0x400000u);
   k.implicit = opaque(0x100000u);
   return k;
 }
@@ -270,13 +277,22 @@ NPBGB_FX_FN L3 from_f64(const Consts& k, uint64_t a, uint64_t b) {
             fma(k.m_base, k.minus_one, pair(x.m, y.m)), fma(k.l_base, k.minus_one, pair(x.l, y.l))};
 }
 
+// Whether from_f64 refused either value.
+NPBGB_FX_FN bool refused_value(const L3& x) {
+  return (first(x.h) << 1) > 0xff000000u || (second(x.h) << 1) > 0xff000000u;
+}
+
 // T rounded in place; returns t's exponent fields, 2^e (in h's scale) of each
 // sum as a binary32 pattern (0 for a zero sum, all ones for NaN).
-NPBGB_FX_FN P2 round_pos(const Consts& k, L3& x) {
-  const P2 t = add_rz(x.h, fma_rz(x.l, k.l_to_m, x.m));
+NPBGB_FX_FN P2 round_pos(const Consts& k, L3& x, P2& t) {
+  t = add_rz(x.h, fma_rz(x.l, k.l_to_m, x.m));
   const P2 e{t.v & kExpBoth};
   x.l = fma(e, k.minus_one, add(x.l, e));
   return e;
+}
+NPBGB_FX_FN P2 round_pos(const Consts& k, L3& x) {
+  P2 t;
+  return round_pos(k, x, t);
 }
 NPBGB_FX_FN P2 round_any(const Consts& k, L3& x) {
   const P2 t1 = add(x.h, x.m);
@@ -296,6 +312,10 @@ NPBGB_FX_FN bool within(uint32_t e) {
   return e - (static_cast<uint32_t>(135 + LO) << 23) < (static_cast<uint32_t>(HI - LO) << 23);
 }
 
+// Whether a sum had an input out of range (NaN), from its exponent fields.
+NPBGB_FX_FN bool refused(uint32_t e) { return e == 0x7f800000u; }
+NPBGB_FX_FN bool refused(P2 e) { return refused(first(e)) || refused(second(e)); }
+
 // A rounded sum of non-negative limbs, 2^-7 <= T < 8, read as T * 2^-(F - 59),
 // in binary64: the limbs' patterns next to a base are integers, their weighted
 // sum is T in units of 2^-59, and dropping the e + 7 low bits (zero after the
@@ -306,12 +326,20 @@ struct Words {
 NPBGB_FX_FN Words words_of(const Consts& k, const L3& x) {
   return Words{add(x.h, k.h_base), add(x.m, k.m_base), add(x.l, k.l_base)};
 }
+// (h << 39) + (m << 19) + l, less the bases; the upper words' part of it.
+constexpr uint64_t kBias = (static_cast<uint64_t>(kHBase) << 39) + (static_cast<uint64_t>(kMBase) << 19);
+static_assert((kBias & 0xffffffffu) == 0, "the bases leave the low word alone");
+
+// The sum as a frame-59 integer, for l >= 0.
+NPBGB_FX_FN int64_t to_fx(uint32_t h, uint32_t m, uint32_t l) {
+  const uint32_t top = h * 128u - static_cast<uint32_t>(kBias >> 32);
+  return static_cast<int64_t>((static_cast<uint64_t>(top) << 32 | (l - kLBase)) +
+                              static_cast<uint64_t>(m) * 0x80000u);
+}
+
 template <int F>
 NPBGB_FX_FN uint64_t to_f64(uint32_t h, uint32_t m, uint32_t l, uint32_t e) {
-  // (h << 39) + (m << 19) + l, less the bases
-  constexpr uint64_t kBias = (static_cast<uint64_t>(kHBase) << 39) + (static_cast<uint64_t>(kMBase) << 19);
   const uint32_t top = h * 128u - static_cast<uint32_t>(kBias >> 32);
-  static_assert((kBias & 0xffffffffu) == 0, "the bases leave the low word alone");
   // l may have been rounded to just below zero: its base comes off with a borrow
   const uint64_t x = (static_cast<uint64_t>(top) << 32 | l) + static_cast<uint64_t>(m) * 0x80000u - kLBase;
   const uint32_t xh = static_cast<uint32_t>(x >> 32), xl = static_cast<uint32_t>(x);
@@ -319,6 +347,63 @@ NPBGB_FX_FN uint64_t to_f64(uint32_t h, uint32_t m, uint32_t l, uint32_t e) {
   const uint32_t lo = shf_r(xl, xh, s);
   const uint32_t hi = shf_r(xh, 0u, s) + (e >> 3) + (static_cast<uint32_t>(946 - F) << 20);
   return static_cast<uint64_t>(hi) << 32 | lo;
+}
+
+NPBGB_FX_FN P2 mul(P2 a, P2 b) {
+#if defined(__CUDA_ARCH__)
+  P2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+#else
+  return each(a, b, b, [](float x, float y, float) { return x * y; });
+#endif
+}
+// The larger magnitude of a and b below c (false if any of them is NaN).
+NPBGB_FX_FN bool both_below(uint32_t a, uint32_t b, uint32_t c) {
+#if defined(__CUDA_ARCH__)
+  return fmaxf(fabsf(__uint_as_float(a)), fabsf(__uint_as_float(b))) < __uint_as_float(c);
+#else
+  const float x = std::fabs(f32_of(a)), y = std::fabs(f32_of(b));
+  return (x > y || y != y ? x : y) < f32_of(c);
+#endif
+}
+
+// RN(0.2 * s) of a rounded sum s of at most five values, with t as round_pos gave
+// it, in limbs that are again non-negative and bounded (m < 2^-19, l < 2^-39: the
+// limbs of five such values still add exactly).  `sure` says for each value whether
+// the result stands; where it does not, it has to be evaluated another way.
+//
+// The double nearest 0.2 is (2^55 + 2) / (5 * 2^55), so the exact product is
+// (s + s * 2^-54) / 5.  Long division of the limbs by five: h from t (so that no
+// carry is left below), then m, each quotient truncated to its grid with a factor
+// just below 1/5, each remainder exact; what is left is l1 = s - 5 (qh + qm), so
+//   product = qh + qm + (l1 + s * 2^-54) / 5.
+// The last term is rounded to a multiple u of the product's last place as in
+// round_any (C = 1.5 * 2^e), from a binary32 estimate (whose error may exceed u/2
+// for the smallest products); its remainder z = l1 - 5 ql + s * 2^-54, exact to
+// 2^-20 u, corrects it, and what is then left of z decides: below 2.5 u (1 - 2^-18)
+// in magnitude the rounding is IEEE's and not a tie.  e is the estimate's exponent,
+// which stands unless the estimate lies within 2^-19 of a power of two: such
+// products, ties, NaN, and products below 2^-7 are not sure.
+NPBGB_FX_FN L3 fifth_of(const Consts& k, const L3& s, P2 t, bool& sure_a, bool& sure_b) {
+  L3 r;
+  r.h = fma(k.h_base, k.minus_one, fma_rz(t, k.fifth, k.h_base));
+  const P2 m1 = add(s.m, fma(k.minus_five, r.h, s.h));
+  r.m = fma(k.m_base, k.minus_one, fma_rz(fma_rz(s.l, k.l_to_m, m1), k.fifth, k.m_base));
+  const P2 l1 = fma(fma(k.minus_five, r.m, m1), k.m_to_l, s.l);
+  const P2 y = mul(fma(t, k.t_to_l, l1), k.fifth);
+  const P2 tr = add_rz(r.h, fma_rz(y, k.l_to_m, r.m));
+  const P2 c = pair(and_or(first(tr), 0x7f800000u, k.half_bit), and_or(second(tr), 0x7f800000u, k.half_bit));
+  const P2 q = fma(c, k.minus_one, add(y, c));
+  const P2 z = fma(t, k.t_to_l, fma(k.minus_five, q, l1));
+  const P2 d = fma(c, k.minus_one, fma(z, k.fifth, c));
+  r.l = add(q, d);
+  const P2 left = mul(fma(k.minus_five, d, z), k.z_scale);
+  const P2 off = fma(c, k.minus_one, tr);
+  const P2 limit = mul(c, k.third);
+  sure_a = both_below(first(left), first(off), first(limit)) && first(c) >= 0x40400000u;
+  sure_b = both_below(second(left), second(off), second(limit)) && second(c) >= 0x40400000u;
+  return r;
 }
 
 }  // namespace fxl
