@@ -185,6 +185,7 @@ struct Consts {
   P2 h_base, m_base, l_base, one, minus_one, l_to_m, h_scale, minus_two, eight;
   P2 fifth, minus_five, m_to_l, t_to_l, z_scale, third;  // (fifth_of)
   uint32_t implicit, half_bit;
+  uint32_t scale = 0;  // the frame holds x * 2^-s: s << 20 (frame_of)
 };
 NPBGB_FX_FN uint32_t opaque(uint32_t v) {
 #if defined(__CUDA_ARCH__)
@@ -264,22 +265,39 @@ NPBGB_FX_FN Bits3 cut_other(uint32_t hi, uint32_t lo) {
 }
 
 NPBGB_FX_FN L3 from_f64(const Consts& k, uint64_t a, uint64_t b) {
-  const uint32_t ah = static_cast<uint32_t>(a >> 32), al = static_cast<uint32_t>(a);
-  const uint32_t bh = static_cast<uint32_t>(b >> 32), bl = static_cast<uint32_t>(b);
+  const uint32_t ah = static_cast<uint32_t>(a >> 32) - k.scale, al = static_cast<uint32_t>(a);
+  const uint32_t bh = static_cast<uint32_t>(b >> 32) - k.scale, bl = static_cast<uint32_t>(b);
   Bits3 x = cut(k, ah, al), y = cut(k, bh, bl);
   // hi words of the range are 0x3f800000 .. 0x3fefffff
   const uint32_t ra = ah - 0x3f800000u, rb = bh - 0x3f800000u;
   if ((ra > rb ? ra : rb) >= 0x700000u) {
-    if (ra >= 0x700000u) x = cut_other(ah, al);
-    if (rb >= 0x700000u) y = cut_other(bh, bl);
+    if (ra >= 0x700000u) x = cut_other(ah + k.scale, al);
+    if (rb >= 0x700000u) y = cut_other(bh + k.scale, bl);
   }
   return L3{fma(k.h_base, k.minus_one, fma_rz(pair(x.h, y.h), k.h_scale, k.h_base)),
             fma(k.m_base, k.minus_one, pair(x.m, y.m)), fma(k.l_base, k.minus_one, pair(x.l, y.l))};
 }
 
+// Consts::scale for values about as large as those sampled: `top` is the largest
+// upper word of their finite non-negative ones.  Binary64 sums and products by
+// constants commute with powers of two while nothing under- or overflows, so a frame
+// may hold x * 2^-s.  Samples in [2^-4, 1) or none keep s = 0; otherwise the frame is
+// [2^-7, 1) times a power of two of two to four times the largest sample.  |s| stays
+// at most 100: then no other value's shifted word looks like one in range, and results
+// stay far from both ends of binary64.
+NPBGB_FX_FN uint32_t frame_of(uint32_t top) {
+  const int e = static_cast<int>(top >> 20) - 1022;
+  const bool keep = top == 0u || (e >= -3 && e <= 0) || e < -101 || e > 99;
+  return keep ? 0u : static_cast<uint32_t>(e + 1) << 20;
+}
+
 // Whether from_f64 refused either value.
 NPBGB_FX_FN bool refused_value(const L3& x) {
   return (first(x.h) << 1) > 0xff000000u || (second(x.h) << 1) > 0xff000000u;
+}
+// Whether it refused both.
+NPBGB_FX_FN bool refused_both(const L3& x) {
+  return (first(x.h) << 1) > 0xff000000u && (second(x.h) << 1) > 0xff000000u;
 }
 
 // T rounded in place; returns t's exponent fields, 2^e (in h's scale) of each
@@ -338,14 +356,14 @@ NPBGB_FX_FN int64_t to_fx(uint32_t h, uint32_t m, uint32_t l) {
 }
 
 template <int F>
-NPBGB_FX_FN uint64_t to_f64(uint32_t h, uint32_t m, uint32_t l, uint32_t e) {
+NPBGB_FX_FN uint64_t to_f64(uint32_t h, uint32_t m, uint32_t l, uint32_t e, uint32_t scale = 0) {
   const uint32_t top = h * 128u - static_cast<uint32_t>(kBias >> 32);
   // l may have been rounded to just below zero: its base comes off with a borrow
   const uint64_t x = (static_cast<uint64_t>(top) << 32 | l) + static_cast<uint64_t>(m) * 0x80000u - kLBase;
   const uint32_t xh = static_cast<uint32_t>(x >> 32), xl = static_cast<uint32_t>(x);
   const uint32_t s = e >> 23;
   const uint32_t lo = shf_r(xl, xh, s);
-  const uint32_t hi = shf_r(xh, 0u, s) + (e >> 3) + (static_cast<uint32_t>(946 - F) << 20);
+  const uint32_t hi = shf_r(xh, 0u, s) + (e >> 3) + (scale + (static_cast<uint32_t>(946 - F) << 20));
   return static_cast<uint64_t>(hi) << 32 | lo;
 }
 

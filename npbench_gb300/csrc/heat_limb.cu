@@ -22,8 +22,12 @@
 // one row in five or one tile in seven (121 and more: binary64 instructions
 // stall the same dispatch).
 //
-// Points whose inputs leave [2^-7, 1) (other than +0) or whose result does are
-// evaluated in hardware binary64 from global memory.
+// The limbs' range is [2^-7, 1), or that times a power of two which the CTA takes from
+// the values at its tile's corners.  NPBench's initial field (values up to 20) then stays
+// in limbs: TSTEPS=11 at 256^3 takes 2.2 ms, in hardware binary64 8.4 and in
+// heat3d_tma 7.8; 25^3, TSTEPS=25, 0.16, 0.26 and 0.39.  Points whose inputs leave the
+// range (other than +0) or whose result does are evaluated in hardware binary64 from
+// global memory.
 #include <cmath>
 
 #include "fxl.cuh"
@@ -83,14 +87,14 @@ __device__ __noinline__ double hardware_point(const double* q, int64_t s0, int64
   return hcore::heat_point<double>(q[0], q[s0], q[-s0], q[s1], q[-s1], q[1], q[-1]);
 }
 
-template <int W, int R>
-__global__ void __launch_bounds__(32 * W, R == 1 ? 6 : 4)
-heat3d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t n0, int64_t n1,
-            int64_t n2, int chunk) {
-  pdl_begin();
+// A CTA's tile and chunk.  SCALED: in the frame that the values at the corners of its
+// first plane (the same for every thread) ask for.  Otherwise in the frame of zero,
+// which costs no instructions, and false (nothing written) if a centre pair of the
+// first plane is out of range.
+template <int W, int R, bool SCALED>
+__device__ __forceinline__ bool run_chunk(const double* __restrict__ src, double* __restrict__ dst, int64_t n0,
+                                          int64_t n1, int64_t n2, int chunk, Plane<W, R> (&plane)[3]) {
   using G = Geom<W, R>;
-  __shared__ Plane<W, R> plane[3];
-  const fxl::Consts K = fxl::consts();
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t k0 = 1 + int64_t(blockIdx.x) * 32, j0 = 1 + int64_t(blockIdx.y) * G::kTileRows;
   const int ib = 1 + int(blockIdx.z) * chunk;
@@ -125,7 +129,6 @@ heat3d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t n0
       x[r].b = in_b[r] ? ld(p, off_b[r]) : 0.5;
     }
   };
-  auto limbs = [&](const Raw& x) { return fxl::from_f64(K, bits_of(x.a), bits_of(x.b)); };
   // The halo of a plane: pair row 0 (the row before the tile and the last row of
   // its first half; warp 0), pair row kRows-1 (warp 1), and the two halo
   // columns (warp 2).
@@ -145,25 +148,49 @@ heat3d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t n0
     x.b = hin_b ? ld(p, hoff_b) : 0.5;
   };
 
+  fxl::Consts K = fxl::consts();
+  auto limbs = [&](const Raw& x) { return fxl::from_f64(K, bits_of(x.a), bits_of(x.b)); };
   Raw own[R], halo{0.5, 0.5};
   L3 x0[R], x1[R], x2[R];
   const double* p = src + int64_t(ib - 1) * s0;
   load_own(p, own);
+  uint32_t corner[4] = {0u, 0u, 0u, 0u};
+  if (SCALED) {
+    const uint32_t last_j = uint32_t((j0 + G::kTileRows < n1 ? j0 + G::kTileRows : n1) - 1 - j0) * uint32_t(n2);
+    const uint32_t last_k = uint32_t((k0 + 32 < n2 ? k0 + 32 : n2) - 1 - k0);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p + s0 + j0 * n2 + k0) + 1;  // upper words
+    corner[0] = q[0];
+    corner[1] = q[2 * last_k];
+    corner[2] = q[2 * last_j];
+    corner[3] = q[2 * (last_j + last_k)];
+  }
+  Raw own1[R];
+  p += s0;
+  load_own(p, own1);
+  if (hr >= 0) load_halo(p, halo);
+  if (SCALED) {
+    uint32_t top = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) top = corner[c] < 0x7ff00000u && corner[c] > top ? corner[c] : top;
+    K.scale = fxl::frame_of(top);
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r) x0[r] = limbs(own[r]);
-  p += s0;
-  load_own(p, own);
-  if (hr >= 0) load_halo(p, halo);
+  bool out_of_range = false;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    x1[r] = limbs(own[r]);
+    x1[r] = limbs(own1[r]);
+    out_of_range = out_of_range || fxl::refused_both(x1[r]);
     plane[0].put(row + r + 1, tx + 1, x1[r]);
   }
   if (hr >= 0) plane[0].put(hr, hc, limbs(halo));
   p += s0;
   load_own(p, own);
   if (hr >= 0 && ib + 1 < ie) load_halo(p, halo);
-  __syncthreads();
+  if (SCALED)
+    __syncthreads();
+  else if (__syncthreads_or(out_of_range))
+    return false;
 
   double* o = dst + int64_t(ib) * s0;
   int i = ib;
@@ -197,9 +224,9 @@ heat3d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t n0
       const P2 e = fxl::round_any(K, w);
       const fxl::Words q = fxl::words_of(K, w);
       double va = __longlong_as_double(
-          fxl::to_f64<62>(fxl::first(q.h), fxl::first(q.m), fxl::first(q.l), fxl::first(e)));
+          fxl::to_f64<62>(fxl::first(q.h), fxl::first(q.m), fxl::first(q.l), fxl::first(e), K.scale));
       double vb = __longlong_as_double(
-          fxl::to_f64<62>(fxl::second(q.h), fxl::second(q.m), fxl::second(q.l), fxl::second(e)));
+          fxl::to_f64<62>(fxl::second(q.h), fxl::second(q.m), fxl::second(q.l), fxl::second(e), K.scale));
       if (!(fxl::within<-4, 3>(fxl::first(e)) && fxl::within<-4, 3>(fxl::second(e)))) {
         const double* g = src + (o - dst);
         if (out_a[r] && !fxl::within<-4, 3>(fxl::first(e))) va = hardware_point(g + off_a[r] / 8, s0, n2);
@@ -216,6 +243,29 @@ heat3d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t n0
   // The register sets and buffers change roles by unrolling, without moves.
   while (step(x0, x1, x2, 0) && step(x1, x2, x0, 1) && step(x2, x0, x1, 2)) {
   }
+  return true;
+}
+
+// Out of line, so that the kernel's registers are the other form's.
+template <int W, int R>
+__device__ __noinline__ void run_scaled(const double* __restrict__ src, double* __restrict__ dst, int64_t n0,
+                                        int64_t n1, int64_t n2, int chunk, Plane<W, R> (&plane)[3]) {
+  run_chunk<W, R, true>(src, dst, n0, n1, n2, chunk, plane);
+}
+
+// With two pairs a thread a CTA tries the frame of zero first: the scale in every
+// conversion costs 3.5% at 256^3.  With one pair that form needs more registers than
+// seven CTAs per SM leave (120^3: 0.605 ms against 0.593, and 0.58 without any scale).
+template <int W, int R>
+__global__ void __launch_bounds__(32 * W, kCtas<R>)
+heat3d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t n0, int64_t n1,
+            int64_t n2, int chunk) {
+  pdl_begin();
+  __shared__ Plane<W, R> plane[3];
+  if constexpr (R == 1)
+    run_chunk<W, R, true>(src, dst, n0, n1, n2, chunk, plane);
+  else if (!run_chunk<W, R, false>(src, dst, n0, n1, n2, chunk, plane))
+    run_scaled<W, R>(src, dst, n0, n1, n2, chunk, plane);
 }
 
 template <int R>

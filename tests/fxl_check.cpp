@@ -113,6 +113,33 @@ int main(int argc, char** argv) {
         ++heats;
       }
     }
+    // the same values in a scaled frame: the same limbs, results scaled back; what no
+    // frame holds stays refused
+    {
+      const int e = int(rng() % 201) - 100;
+      fxl::Consts S = K;
+      S.scale = static_cast<uint32_t>(e) << 20;
+      fxl::L3 w{};
+      for (int i = 0; i < 3; ++i) {
+        w = fxl::from_f64(S, bits_of(std::ldexp(x[i], e)), bits_of(std::ldexp(y[i], e)));
+        if (w.h.v != v[i].h.v || w.m.v != v[i].m.v || w.l.v != v[i].l.v)
+          return fail("scaled frame", x + i, 1, v[i].h.v, w.h.v);
+      }
+      fxl::L3 sum = fxl::add(v[0], v[1]);
+      const fxl::P2 se = fxl::round_pos(K, sum);
+      const fxl::Words o = fxl::words_of(K, sum);
+      if (fxl::within<-7, 3>(fxl::first(se))) {
+        const uint64_t got =
+            fxl::to_f64<59>(fxl::first(o.h), fxl::first(o.m), fxl::first(o.l), fxl::first(se), S.scale);
+        if (got != bits_of(std::ldexp(x[0] + x[1], e))) return fail("scaled sum", x, 2, bits_of(x[0] + x[1]), got);
+      }
+      const double never[] = {-0.0, 5e-324, -0.5, INFINITY, -INFINITY, NAN, 1e-300, -std::ldexp(0.5, e), 1e300,
+                              std::ldexp(1.0, e), std::ldexp(0.0078, e)};
+      const double b = never[it % 11];
+      const fxl::L3 r = fxl::from_f64(S, bits_of(b), bits_of(std::ldexp(0.5, e)));
+      if ((fxl::first(r.h) & 0x7fffffffu) <= 0x7f800000u || (fxl::second(r.h) & 0x7fffffffu) > 0x7f800000u)
+        return fail("scaled refusal", &b, 1, 0, r.h.v);
+    }
     // sums of 3 and 5, in order
     fxl::L3 a = v[0];
     volatile double sx = x[0], sy = y[0];

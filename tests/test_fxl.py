@@ -64,3 +64,32 @@ def test_heat_limbs_at_tile_edges(shape, chunk):
             assert bits_equal(dA.cpu().numpy(), A) and bits_equal(dB.cpu().numpy(), B)
     finally:
         _lib.set_config(_lib.NPBGB_CFG_HEAT_CHUNK, old)
+
+
+# The frame follows the values: NPBench's own initial field, scaled fields, fields whose
+# planes differ by large factors, values beyond any frame; one and two pairs a thread.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(5, 19, 35), (40, 50, 67), (310, 60, 200)])
+@pytest.mark.parametrize("values", ["npbench", "3e3", "2e-13", "steps", "1e200", "awkward"])
+def test_heat_limbs_follow_the_values(shape, values):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from conftest import bits_equal
+    from npbench_gb300 import stencils
+    from oracle import cref
+    rng = np.random.default_rng(3)
+    if values == "npbench":
+        i, j, k = np.indices(shape)
+        A = (i + j + (shape[2] - k)) * 10 / shape[2]
+    elif values == "steps":
+        A = rng.random(shape) * 10.0 ** rng.integers(-40, 40, (shape[0], 1, 1))
+    elif values == "awkward":
+        A = _awkward(shape, 4) * 512
+    else:
+        A = (0.1 + rng.random(shape)) * float(values)
+    B = A[::-1].copy()
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    stencils.heat_3d_kernel(4, dA, dB)
+    cref.heat_3d_kernel(4, A, B)
+    assert bits_equal(dA.cpu().numpy(), A) and bits_equal(dB.cpu().numpy(), B)
