@@ -403,7 +403,7 @@ NPBGB_FX_FN bool both_below(uint32_t a, uint32_t b, uint32_t c) {
 // in magnitude the rounding is IEEE's and not a tie.  e is the estimate's exponent,
 // which stands unless the estimate lies within 2^-19 of a power of two: such
 // products, ties, NaN, and products below 2^-7 are not sure.
-NPBGB_FX_FN L3 fifth_of(const Consts& k, const L3& s, P2 t, bool& sure_a, bool& sure_b) {
+NPBGB_FX_FN L3 fifth_of(const Consts& k, const L3& s, P2 t, bool& sure_a, bool& sure_b, P2& c) {
   L3 r;
   r.h = fma(k.h_base, k.minus_one, fma_rz(t, k.fifth, k.h_base));
   const P2 m1 = add(s.m, fma(k.minus_five, r.h, s.h));
@@ -411,7 +411,7 @@ NPBGB_FX_FN L3 fifth_of(const Consts& k, const L3& s, P2 t, bool& sure_a, bool& 
   const P2 l1 = fma(fma(k.minus_five, r.m, m1), k.m_to_l, s.l);
   const P2 y = mul(fma(t, k.t_to_l, l1), k.fifth);
   const P2 tr = add_rz(r.h, fma_rz(y, k.l_to_m, r.m));
-  const P2 c = pair(and_or(first(tr), 0x7f800000u, k.half_bit), and_or(second(tr), 0x7f800000u, k.half_bit));
+  c = pair(and_or(first(tr), 0x7f800000u, k.half_bit), and_or(second(tr), 0x7f800000u, k.half_bit));
   const P2 q = fma(c, k.minus_one, add(y, c));
   const P2 z = fma(t, k.t_to_l, fma(k.minus_five, q, l1));
   const P2 d = fma(c, k.minus_one, fma(z, k.fifth, c));
@@ -423,6 +423,13 @@ NPBGB_FX_FN L3 fifth_of(const Consts& k, const L3& s, P2 t, bool& sure_a, bool& 
   sure_b = both_below(second(left), second(off), second(limit)) && second(c) >= 0x40400000u;
   return r;
 }
+NPBGB_FX_FN L3 fifth_of(const Consts& k, const L3& s, P2 t, bool& sure_a, bool& sure_b) {
+  P2 c;
+  return fifth_of(k, s, t, sure_a, sure_b, c);
+}
+// Its products in binary64, from the last argument's halves: their exponent fields
+// with the bit below set, which to_f64 only sees in what it adds.
+constexpr uint32_t kFifthScale = 0u - 0x80000u;
 
 }  // namespace fxl
 }  // namespace npbgb

@@ -9,7 +9,8 @@
 // i+1 in registers, w/e neighbours by shuffle, kUnroll rows loaded ahead).
 // Warps never wait on each other.
 //
-// binary32 uses IEEE float operations.  binary64 runs its four additions
+// binary32 uses IEEE float operations.  binary64 runs in binary32 limbs
+// (jacobi_limb.cuh) or, where a setting asks for it, its four additions
 // exactly in fixed point on the integer pipe (fx64.cuh) for every point whose
 // five inputs lie in [2^-7, 1) or are +0 (refused values carry a poison bit),
 // and uses hardware binary64 for any other point.  The fixed-point points also
@@ -17,7 +18,11 @@
 // integer product of the significands, rounded once to nearest even), so they
 // leave the binary64 pipe to the hardware warps.  Both paths give the IEEE
 // result bit for bit.
+#include <algorithm>
+#include <cmath>
+
 #include "jacobi_core.cuh"
+#include "jacobi_limb.cuh"
 #include "tma.cuh"
 
 namespace npbgb {
@@ -91,6 +96,50 @@ jacobi2d_tma(const __grid_constant__ CUtensorMap map, const T* __restrict__ src,
   if (!ok && (threadIdx.x & 31) == 0) atomicOr(&g_jacobi_tma_error, 1u);
 }
 
+template <int W>
+__global__ void __launch_bounds__(32 * W)
+jacobi2d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t ny, int64_t nx, int chunk) {
+  pdl_begin();
+  const int warp = threadIdx.x >> 5;
+  const int64_t k0 = 1 + (int64_t(blockIdx.x) * W + warp) * jlimb::kStrip;
+  if (k0 >= nx - 1) return;
+  const int64_t ib = 1 + int64_t(blockIdx.y) * chunk;
+  const int64_t ie = (ib + chunk < ny - 1) ? ib + chunk : ny - 1;
+  if (!jlimb::rows(jlimb::Limbs{fxl::consts()}, src, dst, nx, k0, ib, ie))
+    jlimb::rows_hardware(src, dst, nx, k0, ib, ie);
+}
+
+// Rows per warp: an even number (two rows at a time), growing with the square root of
+// the strips' rows per warp that the GPU holds at once (36 per SM).  Measured best at
+// q = 0.1 to 2.2: 2 (600^2, TSTEPS=50: 0.425 ms, 4 0.532); 3.3: 4 (1403 x 377: 0.539,
+// 2 0.573, 6 0.652); 6.2: 6 (1000^2: 0.715, 4 0.739, 8 0.795); 15: 8 to 12 (1700 x
+// 1500); 48: 16 (2800^2); 102: 24 (4096^2).
+int limb_chunk(int64_t ny, int64_t nx) {
+  const int64_t least = cdiv(ny - 2, 65535);  // the grid's limit
+  if (g_cfg_jacobi_chunk > 0) return int(std::max<int64_t>(g_cfg_jacobi_chunk, least));
+  const double q = double(cdiv(nx - 2, jlimb::kStrip)) * double(ny - 2) / (36.0 * sm_count());
+  const int64_t pairs = std::max<int64_t>(int64_t(1.2 * std::sqrt(q) + 0.15), 1);
+  return int(std::max<int64_t>(2 * pairs, least + (least & 1)));
+}
+
+// Binary64 in limbs (jacobi_limb.cuh).  Bound by instructions on large grids, by a
+// launch's latency on small ones.  Against the fixed-point strips and the TMA ring
+// with their best settings (ms, TSTEPS=50, 11 at 2800^2 and 4096^2; then NPBench's
+// initial field, whose values leave [0, 1)): 300^2 0.356 to 0.29 and 0.49 to 0.34;
+// 1000^2 0.84 to 0.715 and 1.31 to 0.74; 2800^2 0.95 to 0.80 and 1.80 to 0.81; 4096^2
+// 1.71 to 1.48 and 3.41 to 1.49.
+int32_t run_limb(double* a, double* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st) {
+  constexpr int W = 4;
+  const int chunk = limb_chunk(ny, nx);
+  const dim3 grid{unsigned(cdiv(nx - 2, W * jlimb::kStrip)), unsigned(cdiv(ny - 2, chunk))};
+  cudaError_t e = cudaSuccess;
+  for (int32_t t = 1; t < tsteps && e == cudaSuccess; ++t) {
+    e = launch_chained(jacobi2d_limb<W>, grid, dim3{32u * W}, 0, st, a, b, ny, nx, chunk);
+    if (e == cudaSuccess) e = launch_chained(jacobi2d_limb<W>, grid, dim3{32u * W}, 0, st, b, a, ny, nx, chunk);
+  }
+  return cuda_status(e, "jacobi2d_limb");
+}
+
 int pick_chunk(int64_t ny, int64_t col_blocks) {
   if (g_cfg_jacobi_chunk > 0) return int(g_cfg_jacobi_chunk);
   // About 16 warps per SM over 152 SMs, rows per warp at least 3 (small
@@ -136,6 +185,12 @@ int32_t run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st)
   {
     const int32_t r = jacobi2d_bands_run<T>(a, b, ny, nx, tsteps, st);
     if (r != NPBGB_ERR_STATE) return r;
+  }
+  if constexpr (FX) {
+    // Limbs unless a setting of the other forms asks for one of those.
+    if (g_cfg_jacobi_hw_warps < 0 && g_cfg_jacobi_tma != 2 && g_cfg_jacobi_fx_adds == 0 &&
+        g_cfg_jacobi_fx_mul == 1)
+      return run_limb(a, b, ny, nx, tsteps, st);
   }
   const int64_t gx = cdiv(nx - 2, 32 * kWarps);
   const int chunk = pick_chunk(ny, gx);

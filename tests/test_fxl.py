@@ -93,3 +93,46 @@ def test_heat_limbs_follow_the_values(shape, values):
     stencils.heat_3d_kernel(4, dA, dB)
     cref.heat_3d_kernel(4, A, B)
     assert bits_equal(dA.cpu().numpy(), A) and bits_equal(dB.cpu().numpy(), B)
+
+
+# Jacobi-2D in limbs, one launch per half-sweep: strips of 30 columns, four to a CTA, two
+# row ranges of which the second may be one short; fields in and out of the frame.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(3, 3), (4, 32), (5, 33), (9, 122), (34, 123), (65, 62)])
+@pytest.mark.parametrize("values", ["unit", "npbench", "awkward", "signed", "hot_wall", "steps"])
+def test_jacobi_limbs_at_strip_edges(shape, values):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from conftest import bits_equal
+    from npbench_gb300 import _lib, stencils
+    from oracle import cref
+    rng = np.random.default_rng(7)
+    A = rng.random(shape)
+    if values == "npbench":
+        i, j = np.indices(shape)
+        A = i * (j + 2) / shape[0]
+    elif values == "awkward":
+        A = _awkward(shape, 5)
+    elif values == "signed":
+        A = rng.standard_normal(shape)
+    elif values == "hot_wall":
+        A = np.zeros(shape)
+        A[0] = 100.0
+    elif values == "steps":
+        A = A * 10.0 ** rng.integers(-40, 40, (shape[0], 1))
+    B = A[::-1].copy()
+    old = [(k, _lib.set_config(k, v)) for k, v in ((_lib.NPBGB_CFG_JACOBI_BANDS, 0),
+                                                   (_lib.NPBGB_CFG_JACOBI_CHUNK, 0))]
+    try:
+        for chunk in (0, 1, 5):
+            _lib.set_config(_lib.NPBGB_CFG_JACOBI_CHUNK, chunk)
+            a, b = A.copy(), B.copy()
+            dA, dB = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+            stencils.jacobi_2d_kernel(6, dA, dB)
+            with np.errstate(all="ignore"):
+                cref.jacobi_2d_kernel(6, a, b)
+            assert bits_equal(dA.cpu().numpy(), a) and bits_equal(dB.cpu().numpy(), b)
+    finally:
+        for k, v in old:
+            _lib.set_config(k, v)
