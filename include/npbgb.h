@@ -74,7 +74,8 @@ extern "C" {
                                          time loops use programmatic dependent launch;
                                          0: plain stream order */
 #define NPBGB_CFG_BATCH_MODE 11       /* form of a batch, read when it is planned:
-                                         0 (default) automatic by size, 1 persistent,
+                                         0 (default) automatic (stepped, but for small
+                                         batches of very many steps), 1 persistent,
                                          2 stepped, 3 queue (NPBGB_BATCH_*) */
 #define NPBGB_CFG_HDIFF_EMU 12        /* hdiff: which Laplacian and flux items run on the
                                          integer pipes (exact binary64 addition in
@@ -339,20 +340,20 @@ NPBGB_API int32_t npbgb_channel_flow(void* u, void* v, void* p, int64_t ny, int6
                                      void* workspace, int64_t workspace_bytes, int64_t* steps,
                                      void* stream);
 
-/* Batches: many independent grids advanced by one persistent launch.
+/* Batches: many independent grids advanced together.
  *
  * npbgb_batch_create plans a batch of Jacobi-2D and Heat-3D grids: each grid
  * is cut along axis 0 into bands (the grid's band_rows, else band_rows, else
- * the kind's default), bands are assigned
- * to the CTAs of one cooperative launch with equal work per CTA, and the
- * plan (band table, per-band step counters) is stored in device memory
- * allocated here.  Each grid ends exactly as npbgb_jacobi2d / npbgb_heat3d
+ * rows that follow the batch), and the plan is stored in device memory
+ * allocated here: tables of the tiles of each half-sweep's launch (stepped
+ * form), or the bands of the CTAs of one cooperative launch with equal work
+ * per CTA and their step counters (persistent form).  Each grid ends exactly as npbgb_jacobi2d / npbgb_heat3d
  * would leave it (bit-identical), i.e. as the reference's kernel(TSTEPS, A, B)
  * per grid, polybench/jacobi_2d/jacobi_2d_numpy.py:4-10 and
  * polybench/heat_3d/heat_3d_numpy.py:4-20.
- * npbgb_batch_launch runs the whole batch: a counter reset and one
- * persistent kernel on `stream`; with use_graph != 0 the two are captured
- * once into a CUDA graph and replayed.  Bounded waits: a CTA that makes no
+ * npbgb_batch_launch runs the whole batch on `stream`: one launch per
+ * half-sweep, or a counter reset and one persistent kernel; with use_graph
+ * != 0 they are captured once into a CUDA graph and replayed.  Bounded waits: a CTA that makes no
  * progress for two seconds records an error reported by npbgb_device_status.
  * The grids' arrays must stay allocated while the batch is in use. */
 NPBGB_API int32_t npbgb_batch_create(const npbgb_grid* grids, int64_t count, int32_t band_rows,

@@ -1,11 +1,11 @@
-"""Many independent grids advanced by one persistent launch (libnpbgb batches).
+"""Many independent grids advanced together (libnpbgb batches).
 
     with Batch([(A0, B0, T0), (A1, B1, T1), ...]) as batch:
-        batch.launch()              # one counter reset + one cooperative persistent kernel
+        batch.launch()              # one chained launch per half-sweep over all grids still active
         batch.launch(graph=True)    # the same, captured once into a CUDA graph and replayed
 
-Batches of 2^24 cells or more run in the stepped form (one chained launch per
-half-sweep over all grids still active), smaller ones in the persistent form;
+That is the stepped form; small batches (under 2^24 cells) of more than 16384
+half-sweeps run in the persistent form, one cooperative launch for all of them;
 ``mode="queue"`` runs the batch as one launch of the device-side tile work
 queue, and NPBGB_CFG_BATCH_MODE or ``mode`` forces any form.  ``guard=True``
 runs float32 grids whose float32 error would exceed NPBench's bound in float64

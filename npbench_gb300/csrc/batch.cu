@@ -20,15 +20,22 @@
 // polybench/jacobi_2d/jacobi_2d_numpy.py:6-10), including the fixed-point
 // binary64 path.
 //
-// Large batches take a second form ("stepped"): one launch per half-sweep
+// By default batches take a second form ("stepped"): one launch per half-sweep
 // index s covers every tile of every grid that still has a half-sweep s to do,
 // and consecutive launches are chained (programmatic dependent launch), so the
 // kernel boundary is the only dependency and no CTA ever waits on another.
 // Grids are sorted by their half-sweep count, so the grids active at s are a
 // prefix and launch s simply covers the first N_s tiles; a tile table maps each
-// CTA to its grid.  Small batches keep the persistent form, whose launch count
-// does not grow with the step count.
+// CTA to its grid.  The persistent form's launch count does not grow with the
+// step count; it takes over for small batches of very many steps.
+//
+// Bound by the latency of a launch and a unit's rows where few grids are active, by the
+// limbs' instructions where many are.  Measured (one pass as a graph, binary32 grids
+// promoted; before limbs, flattened units and rows by phase): 32 grids of 64 to 2048 a
+// side with up to 998 half-sweeps 42.9 to 22.2 ms, 8 of them 21.6 to 5.8 ms, 32 of 64 to
+// 256 18.7 to 4.8 ms, 200 grids 184 to 129 ms.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -38,6 +45,7 @@
 
 #include "heat_core.cuh"
 #include "jacobi_core.cuh"
+#include "jacobi_limb.cuh"
 #include "npbgb_common.cuh"
 #include "queue.cuh"
 #include "tma.cuh"
@@ -78,7 +86,8 @@ struct StepGrid {
   int32_t step0;       // half-sweeps already done (parity of the first source)
   int32_t count;       // half-sweeps to do in this launch chain
   int32_t chunk;       // rows (Jacobi-2D) or planes (Heat-3D) per tile
-  int32_t tx, ty;      // tiles along the contiguous axis and the next one
+  int32_t tx, ty;      // tiles along the contiguous axis and the next one; Jacobi-2D in
+                       // the limb kernel: column strips, and their width (30: limbs)
   int16_t dtype, kind;
   int32_t map;         // binary64 Jacobi-2D: index of the grid's tensor-map pair, or -1
 };
@@ -219,13 +228,21 @@ batch_persistent(const BandDesc* __restrict__ bands, uint32_t* done, const int32
   }
 }
 
-// Half-sweep s of every tile in [0, gridDim.x): CTA t finds its grid in the
-// tile table and processes one tile (Jacobi-2D: 8 warps x 32 columns x chunk
-// rows; Heat-3D: a 32 x 8 column tile streamed over chunk planes).  Five CTAs
-// per SM (48 registers, a few spilled): on the 4096-grid batch 3.13 s per pass
-// against 3.36 s with four (64 registers) and 3.47 s with six (40 registers,
-// more spills).
-__global__ void __launch_bounds__(kBThreads, 5)
+// Half-sweep s of every tile in [0, gridDim.x): CTA t finds its grid in the tile table
+// and processes one tile.  Heat-3D: a 32 x 8 column tile streamed over chunk planes.
+//
+// LIMB (most work is Jacobi-2D): binary64 Jacobi-2D in limbs (jacobi_limb.cuh; four
+// CTAs per SM).  A Jacobi-2D tile is eight units of one strip of columns x chunk rows,
+// a warp each, numbered along the rows of strips, so that a grid's last tile alone has
+// idle warps.
+//
+// Otherwise (mostly Heat-3D, whose tiles want five CTAs per SM: 32 grids of 120^3, 20.7
+// ms against 22.8; or a setting asks for hardware warps or the TMA rings): a Jacobi-2D
+// tile is 8 warps x 32 columns x chunk rows, binary64 in fixed point.  48 registers, a
+// few spilled: on the 4096-grid batch 3.13 s per pass against 3.36 s with four CTAs (64
+// registers) and 3.47 s with six (40 registers, more spills).
+template <bool LIMB>
+__global__ void __launch_bounds__(kBThreads, LIMB ? 4 : 5)
 batch_step(const StepGrid* __restrict__ grids, const int32_t* __restrict__ tile_grid, int32_t s,
            int f64_emulation, int hw_warps, uint32_t one, const CUtensorMap* __restrict__ maps) {
   pdl_begin();
@@ -259,6 +276,22 @@ batch_step(const StepGrid* __restrict__ grids, const int32_t* __restrict__ tile_
     return;
   }
   const int warp = threadIdx.x >> 5;
+  if constexpr (LIMB) {
+    const int64_t unit = r * kBWarps + warp;
+    const int64_t k0 = 1 + unit % G.tx * G.ty;
+    const int64_t ib = 1 + unit / G.tx * G.chunk, ie = min(ib + G.chunk, int64_t(G.n0) - 1);
+    if (ib >= ie) return;  // warp-uniform; no CTA barrier here
+    if (G.dtype == NPBGB_F64) {
+      const double* sp = static_cast<const double*>(src);
+      double* dp = static_cast<double*>(dst);
+      if (!f64_emulation || !jlimb::rows(jlimb::Limbs{fxl::consts()}, sp, dp, G.n1, k0, ib, ie))
+        jlimb::rows_hardware(sp, dp, G.n1, k0, ib, ie);
+    } else {
+      jcore::strip_rows<float, false, false, 4>(static_cast<const float*>(src), static_cast<float*>(dst), G.n1, k0,
+                                                ib, ie, one);
+    }
+    return;
+  }
   const int64_t k0 = 1 + (bx * kBWarps + warp) * 32;
   if (k0 >= G.n1 - 1) return;  // warp-uniform; the strip path has no CTA barrier
   const int64_t ib = 1 + rest * G.chunk, ie = min(ib + G.chunk, int64_t(G.n0) - 1);
@@ -356,7 +389,10 @@ struct npbgb_batch {
   npbgb::StepGrid* d_step = nullptr;
   int32_t* d_tiles = nullptr;
   int64_t cap_step = 0, cap_tiles = 0, ntiles = 0;
-  std::vector<int32_t> launch_tiles;  // CTAs of launch s = tiles of the grids active at s
+  // A launch: its tiles (those of the grids active at s) and where its phase's tables begin.
+  struct Launch { int32_t tiles; int64_t grids_at, tiles_at; };
+  std::vector<Launch> launches;
+  bool limb = false;  // planned for the limb kernel
   npbgb::ConvChunk* d_conv = nullptr;  // stepped form: conversion chunks of promoted grids
   int64_t cap_conv = 0, nconv = 0;
   CUtensorMap* d_maps = nullptr;  // stepped form: tensor maps (a, b) of the TMA grids
@@ -458,10 +494,14 @@ int32_t launch_stepped(npbgb_batch* b, cudaStream_t st) {
   if (b->nconv > 0)
     e = launch_chained(batch_convert, dim3{unsigned(b->nconv)}, dim3{256u}, 0, st,
                        static_cast<const ConvChunk*>(b->d_conv), 1);
-  for (size_t s = 0; s < b->launch_tiles.size() && e == cudaSuccess; ++s)
-    e = launch_chained(batch_step, dim3{unsigned(b->launch_tiles[s])}, dim3{unsigned(kBThreads)},
-                       b->step_smem, st, b->d_step, b->d_tiles, int32_t(s), f64_emul, hw_warps, 1u,
+  const auto kern = b->limb ? batch_step<true> : batch_step<false>;
+  for (size_t s = 0; s < b->launches.size() && e == cudaSuccess; ++s) {
+    const npbgb_batch::Launch& l = b->launches[s];
+    e = launch_chained(kern, dim3{unsigned(l.tiles)}, dim3{unsigned(kBThreads)}, b->step_smem, st,
+                       static_cast<const StepGrid*>(b->d_step + l.grids_at),
+                       static_cast<const int32_t*>(b->d_tiles + l.tiles_at), int32_t(s), f64_emul, hw_warps, 1u,
                        static_cast<const CUtensorMap*>(b->d_maps));
+  }
   if (b->nconv > 0 && e == cudaSuccess)
     e = launch_chained(batch_convert, dim3{unsigned(b->nconv)}, dim3{256u}, 0, st,
                        static_cast<const ConvChunk*>(b->d_conv), 0);
@@ -496,9 +536,26 @@ int32_t launch_batch(npbgb_batch* b, cudaStream_t st) {
 
 namespace {
 
-// Batches of at least this many cells take the stepped form by default: each
-// half-sweep launch then has enough tiles to fill the GPU many times over.
+// Batches take the stepped form by default, at every size (200 steps, stepped against
+// persistent: one 64^2 grid 1.1 against 6.0 ms, eight of 64 to 2048 a side 5.5 against
+// 52.0), unless a small one has so many half-sweeps that a graph of its launches would
+// be costly to build: then the persistent form's single launch.
 constexpr int64_t kSteppedCells = int64_t(1) << 24;
+constexpr int64_t kSteppedLaunches = 16384;
+
+// Rows per unit for the first `active` grids: jacobi2d.cu's rule, with 32 warps per SM,
+// in steps that keep the phases few.
+int32_t step_chunk(const std::vector<npbgb::StepGrid>& sg, size_t active, bool limb) {
+  double rows = 0.0;
+  for (size_t q = 0; q < active; ++q)
+    if (sg[q].kind != NPBGB_KIND_HEAT3D) rows += double(sg[q].tx) * double(sg[q].n0 - 2);
+  if (!limb) rows *= npbgb::kBWarps;
+  const double want = 2.0 * (1.2 * std::sqrt(rows / (32.0 * npbgb::sm_count())) - 0.35);
+  int32_t chunk = 2;
+  for (const int32_t c : {4, 6, 8, 12, 16, 24, 32, 48})
+    if (want > 0.8 * c) chunk = c;
+  return chunk;
+}
 
 // The stepped form of `grids` (already validated by plan_grid).
 int32_t plan_stepped(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int32_t band_rows,
@@ -506,6 +563,13 @@ int32_t plan_stepped(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int
   using namespace npbgb;
   std::vector<StepGrid> sg;
   std::vector<CUtensorMap> maps;
+  double jacobi = 0.0, heat3d = 0.0;  // updates
+  for (int64_t g = 0; g < count; ++g) {
+    const npbgb_grid& G = grids[g];
+    const bool heat = G.kind == NPBGB_KIND_HEAT3D;
+    (heat ? heat3d : jacobi) += double(G.n0) * double(G.n1) * (heat ? double(G.n2) : 1.0) * double(G.tsteps);
+  }
+  const bool limb = jacobi > heat3d && g_cfg_jacobi_hw_warps < 0 && !g_cfg_batch_tma && g_cfg_f64_emulation;
   for (int64_t g = 0; g < count; ++g) {
     const npbgb_grid& G = grids[g];
     const bool heat = G.kind == NPBGB_KIND_HEAT3D;
@@ -541,14 +605,13 @@ int32_t plan_stepped(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int
         maps.push_back(mb);
       }
     }
-    const int32_t rows = G.band_rows > 0 ? G.band_rows : (band_rows > 0 ? band_rows : (heat ? 16 : 32));
-    d.chunk = rows;
+    d.chunk = G.band_rows > 0 ? G.band_rows : (band_rows > 0 ? band_rows : (heat ? 16 : 0));
     if (heat) {
       d.tx = int32_t(cdiv(G.n2 - 2, hcore::kTK));
       d.ty = int32_t(cdiv(G.n1 - 2, hcore::kTJ));
     } else {
-      d.tx = int32_t(cdiv(G.n1 - 2, 32 * kBWarps));
-      d.ty = 1;
+      d.ty = limb ? (G.dtype == NPBGB_F64 ? jlimb::kStrip : 32) : 1;
+      d.tx = int32_t(cdiv(G.n1 - 2, limb ? d.ty : 32 * kBWarps));
     }
     sg.push_back(d);
   }
@@ -570,27 +633,49 @@ int32_t plan_stepped(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int
   if (int64_t(conv.size()) > 0x7fffffff) return set_error(NPBGB_ERR_NOMEM, "batch: too many chunks");
   std::stable_sort(sg.begin(), sg.end(),
                    [](const StepGrid& x, const StepGrid& y) { return x.count > y.count; });
+  // Launch s covers the grids with count > s: a prefix of the sorted list.  Rows per
+  // unit that the caller left open follow the grids still active, as in jacobi2d.cu
+  // (few grids want short units, many long ones), in phases with tables of their own.
+  std::vector<StepGrid> tables;
   std::vector<int32_t> tiles;
-  for (size_t q = 0; q < sg.size(); ++q) {
-    StepGrid& d = sg[q];
-    const int64_t n = int64_t(d.tx) * d.ty * cdiv(int64_t(d.n0) - 2, d.chunk);
-    d.first_tile = int64_t(tiles.size());
-    if (int64_t(tiles.size()) + n > 0x7fffffff) return set_error(NPBGB_ERR_NOMEM, "batch: too many tiles");
-    tiles.insert(tiles.end(), size_t(n), int32_t(q));
-  }
-  // Launch s covers the grids with count > s: a prefix of the sorted list.
-  std::vector<int32_t> launch_tiles;
+  std::vector<npbgb_batch::Launch> launches;
   {
     size_t active = sg.size();
     const int32_t smax = sg.empty() ? 0 : sg.front().count;
+    int32_t chunk = 0;        // of the phase
+    bool open = false;        // whether any grid follows it
+    for (const StepGrid& d : sg) open = open || d.chunk == 0;
+    int64_t grids_at = 0, tiles_at = 0;
+    size_t last_active = 0;
     for (int32_t st = 0; st < smax; ++st) {
       while (active > 0 && sg[active - 1].count <= st) --active;
-      launch_tiles.push_back(int32_t(active == sg.size() ? int64_t(tiles.size())
-                                                         : sg[active].first_tile));
+      if (st == 0 || (open && active != last_active)) {
+        const int32_t want = step_chunk(sg, active, limb);
+        if (st == 0 || want < chunk) {
+          chunk = want;
+          grids_at = int64_t(tables.size());
+          tiles_at = int64_t(tiles.size());
+          for (size_t q = 0; q < active; ++q) {
+            StepGrid d = sg[q];
+            if (d.chunk == 0) d.chunk = chunk;
+            const int64_t units = int64_t(d.tx) * cdiv(int64_t(d.n0) - 2, d.chunk);
+            const int64_t n = limb && d.kind != NPBGB_KIND_HEAT3D ? cdiv(units, kBWarps) : units * d.ty;
+            d.first_tile = int64_t(tiles.size()) - tiles_at;
+            if (int64_t(tiles.size()) + n > 0x7fffffff) return set_error(NPBGB_ERR_NOMEM, "batch: too many tiles");
+            tiles.insert(tiles.end(), size_t(n), int32_t(q));
+            tables.push_back(d);
+          }
+        }
+        last_active = active;
+      }
+      const int64_t end = grids_at + int64_t(active) < int64_t(tables.size())
+                              ? tables[size_t(grids_at) + active].first_tile
+                              : int64_t(tiles.size()) - tiles_at;
+      launches.push_back({int32_t(end), grids_at, tiles_at});
     }
   }
   cudaError_t e;
-  const int64_t need_step = std::max<int64_t>(1, int64_t(sg.size()));
+  const int64_t need_step = std::max<int64_t>(1, int64_t(tables.size()));
   if (need_step > b->cap_step) {
     cudaFree(b->d_step);
     b->d_step = nullptr;
@@ -609,7 +694,7 @@ int32_t plan_stepped(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int
     b->cap_tiles = need_tiles;
   }
   if (!sg.empty() &&
-      ((e = cudaMemcpy(b->d_step, sg.data(), sizeof(StepGrid) * sg.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
+      ((e = cudaMemcpy(b->d_step, tables.data(), sizeof(StepGrid) * tables.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
        (e = cudaMemcpy(b->d_tiles, tiles.data(), sizeof(int32_t) * tiles.size(), cudaMemcpyHostToDevice)) != cudaSuccess))
     return cuda_status(e, "batch: upload");
   if (int64_t(conv.size()) > b->cap_conv) {
@@ -637,10 +722,11 @@ int32_t plan_stepped(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int
     return cuda_status(e, "batch: upload");
   b->step_smem = maps.empty() ? 0 : jcore::TmaStrip<double, kBWarps>::smem() + 128;
   b->mode = NPBGB_BATCH_STEPPED;
-  b->ntiles = int64_t(tiles.size());
-  b->launch_tiles = std::move(launch_tiles);
+  b->limb = limb;
+  b->ntiles = launches.empty() ? 0 : launches.front().tiles;
+  b->launches = std::move(launches);
   b->nbands = b->ntiles;  // "nothing to do" checks use nbands
-  b->nctas = int(b->launch_tiles.size());
+  b->nctas = int(b->launches.size());
   b->updates = updates;
   return NPBGB_OK;
 }
@@ -651,9 +737,11 @@ int32_t plan_into(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int32_
   using namespace npbgb;
   if (count < 0 || (count > 0 && !grids)) return set_error(NPBGB_ERR_ARG, "batch: bad grid list");
   if (band_rows < 0) return set_error(NPBGB_ERR_ARG, "batch: band_rows < 0");
-  int64_t cells = 0;
+  int64_t cells = 0, launches = 0;
   for (int64_t g = 0; g < count; ++g) {
     const npbgb_grid& G = grids[g];
+    const int64_t todo = 2 * (int64_t(G.tsteps) - 1) - G.step0;
+    launches = std::max(launches, G.nsteps > 0 ? std::min<int64_t>(G.nsteps, todo) : todo);
     cells += int64_t(G.n0) * G.n1 * (G.kind == NPBGB_KIND_HEAT3D ? G.n2 : 1);
   }
   bool conv = false;
@@ -662,8 +750,9 @@ int32_t plan_into(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int32_
   // which the stepped and queue forms have; by default they take the stepped one.
   const int32_t mode = g_cfg_batch_mode != 0
                            ? int32_t(g_cfg_batch_mode)
-                           : ((conv || cells >= kSteppedCells) ? NPBGB_BATCH_STEPPED
-                                                               : NPBGB_BATCH_PERSISTENT);
+                           : ((conv || cells >= kSteppedCells || launches <= kSteppedLaunches)
+                                  ? NPBGB_BATCH_STEPPED
+                                  : NPBGB_BATCH_PERSISTENT);
   if (mode == NPBGB_BATCH_QUEUE) {
     // The queue planner validates the grids itself (it also takes binary32
     // arrays of grids run in binary64).
@@ -679,7 +768,7 @@ int32_t plan_into(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int32_
     qhost::free_static(b->sq);
     b->sq = sq;
     b->mode = NPBGB_BATCH_QUEUE;
-    b->launch_tiles.clear();
+    b->launches.clear();
     b->ntiles = qtiles;
     b->nbands = qtiles;  // "nothing to do" checks use nbands
     b->nctas = qhost::static_ctas(b->sq);
@@ -706,7 +795,7 @@ int32_t plan_into(npbgb_batch* b, const npbgb_grid* grids, int64_t count, int32_
   b->nconv = 0;
   if (mode == NPBGB_BATCH_STEPPED) return plan_stepped(b, grids, count, band_rows, updates);
   b->mode = NPBGB_BATCH_PERSISTENT;
-  b->launch_tiles.clear();
+  b->launches.clear();
   int per_sm = 0;
   const int ctas_per_sm = int(g_cfg_batch_ctas_per_sm);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_kernel(ctas_per_sm), kBThreads, 0);

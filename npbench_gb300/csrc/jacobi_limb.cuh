@@ -29,7 +29,7 @@ using fxl::P2;
 __device__ __forceinline__ double hardware(double c, double w, double e, double s, double n) {
   return mul_rn(0.2, add_rn(add_rn(add_rn(add_rn(c, w), e), s), n));
 }
-__device__ __noinline__ double hardware_point(const double* p, int64_t nx) {
+static __device__ __noinline__ double hardware_point(const double* p, int64_t nx) {
   return hardware(p[0], p[-1], p[1], p[nx], p[-nx]);
 }
 
@@ -149,7 +149,7 @@ __device__ __forceinline__ bool rows(M m, const double* __restrict__ src, double
   return true;
 }
 
-__device__ __noinline__ void rows_hardware(const double* __restrict__ src, double* __restrict__ dst, int64_t nx,
+static __device__ __noinline__ void rows_hardware(const double* __restrict__ src, double* __restrict__ dst, int64_t nx,
                                            int64_t k0, int64_t r0, int64_t r1) {
   rows(Hardware{}, src, dst, nx, k0, r0, r1);
 }
