@@ -16,7 +16,10 @@
 // heat3d_ldg (any layout): each plane tile is staged by plain loads into
 //   three rotating shared buffers; axis-0 neighbours stay in registers.
 //
-// binary32 uses IEEE float operations.  binary64 runs in fixed point on the
+// By default binary32 runs in heat_rows.cu and binary64 in heat_limb.cu; the
+// forms here take over where a setting asks for them or those refuse.
+//
+// binary32 uses IEEE float operations.  binary64 here runs in fixed point on the
 // integer pipe (fx64.cuh): staged values are converted once to frame-59
 // integers, values outside [2^-7, 1) (other than +0) are marked with a poison
 // bit, and a point whose seven inputs are all clean is evaluated with exact
@@ -43,6 +46,8 @@ extern int64_t g_cfg_heat_stages;
 extern int64_t g_cfg_heat_mad_rows;
 
 int32_t heat3d_limb_run(double* a, double* b, int64_t n0, int64_t n1, int64_t n2, int32_t tsteps,
+                        cudaStream_t st);
+int32_t heat3d_rows_run(float* a, float* b, int64_t n0, int64_t n1, int64_t n2, int32_t tsteps,
                         cudaStream_t st);
 int32_t heat3d_tb2_run(float* a, float* b, int64_t n0, int64_t n1, int64_t n2, int32_t tsteps,
                        cudaStream_t st, int32_t (*single_pairs)(float*, float*, int64_t, int64_t,
@@ -402,6 +407,16 @@ int32_t run_single(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tstep
       if (r != NPBGB_ERR_STATE) return r;
     }
   }
+  // binary32 streams rows with plain loads (heat_rows.cu) unless a setting of the TMA
+  // form is made and TMA can copy the arrays: faster at every size measured (ms,
+  // rows / TMA / staged: 64^3, TSTEPS=50, 0.26 / 0.38 / -; 224^3, 21, 0.64 / 0.72; 310 x
+  // 311 x 319, 11, 0.98 / - / 3.44) but 512^3 (5: 1.59 / 1.55).
+  if constexpr (sizeof(T) == 4) {
+    if (!g_cfg_heat_tma || (g_cfg_heat_rows == 0 && g_cfg_heat_stages == 0)) {
+      const int32_t r = heat3d_rows_run(a, b, n0, n1, n2, tsteps, st);
+      if (r != NPBGB_ERR_STATE) return r;
+    }
+  }
   if (g_cfg_heat_tma) {
     // Tuned on GB300 (256^3): binary32 is memory-latency bound and wants more
     // rows per thread; binary64 (integer-pipe bound) wants one.
@@ -428,6 +443,10 @@ int32_t run_single(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tstep
     else
       r = cvt ? launch_tma<T, FX, 1, true>(a, b, n0, n1, n2, tsteps, st)
               : launch_tma<T, FX, 1, false>(a, b, n0, n1, n2, tsteps, st);
+    if (r != NPBGB_ERR_STATE) return r;
+  }
+  if constexpr (sizeof(T) == 4) {
+    const int32_t r = heat3d_rows_run(a, b, n0, n1, n2, tsteps, st);
     if (r != NPBGB_ERR_STATE) return r;
   }
   return launch_ldg<T, FX>(a, b, n0, n1, n2, tsteps, st);
