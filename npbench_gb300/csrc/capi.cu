@@ -52,6 +52,7 @@ uint32_t take_cfd_device_error();
 uint32_t take_queue_device_error();
 uint32_t take_heat_tb_device_error();
 uint32_t take_jacobi_bands_device_error();
+uint32_t take_jacobi1d_device_error();
 uint32_t take_jacobi_tma_device_error();
 int32_t launch_wait_timeout_selftest(uint64_t limit_ns, cudaStream_t st);
 
@@ -281,7 +282,7 @@ int32_t npbgb_device_status(void* stream) {
   if (e != cudaSuccess) return cuda_status(e, "device status");
   const uint32_t h = take_heat_device_error() | take_heat_tb_device_error();
   const uint32_t bt = take_batch_device_error();
-  const uint32_t cf = take_cfd_device_error() | take_jacobi_bands_device_error();
+  const uint32_t cf = take_cfd_device_error() | take_jacobi_bands_device_error() | take_jacobi1d_device_error();
   const uint32_t jt = take_jacobi_tma_device_error();
   const uint32_t qu = take_queue_device_error();
   if (h == 0xffffffffu || bt == 0xffffffffu || cf == 0xffffffffu || qu == 0xffffffffu || jt == 0xffffffffu)

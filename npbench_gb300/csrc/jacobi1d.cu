@@ -29,6 +29,7 @@ extern int64_t g_cfg_jacobi1d_ctas;
 extern int64_t g_cfg_jacobi1d_depth;
 int64_t jacobi1d_effective_depth();
 int64_t jacobi1d_effective_ctas();
+int32_t jacobi1d_resident_run(float* a, float* b, int64_t n, int32_t tsteps, cudaStream_t st);
 
 namespace {
 
@@ -38,6 +39,8 @@ constexpr int kMaxDepth = 64;
 // / 64 with one CTA per SM 3.72 / 3.19 / 3.13 / 3.18.  More CTAs per SM add
 // halo work without gaining speed (2 per SM 3.62 without PDL).
 constexpr int kDefaultDepth = 48, kDefaultCtas = 1;
+// N=34000: TSTEPS=51 46 us resident against 48 chained, 101 57 against 63, 401 111 against 162.
+constexpr int kLeastResident = 64;
 
 template <typename T>
 __global__ void __launch_bounds__(kMaxThreads)
@@ -83,6 +86,14 @@ jacobi1d_block(T* __restrict__ a, T* __restrict__ b, int64_t n, int steps, int w
 template <typename T>
 int32_t run(T* a, T* b, int64_t n, int32_t tsteps, cudaStream_t st) {
   if (tsteps <= 1 || n < 3) return NPBGB_OK;
+  // binary32 hands values on within one launch (jacobi1d_resident.cu) unless a setting
+  // of the chained form is made; runs of a few chained launches are faster chained.
+  if constexpr (sizeof(T) == 4) {
+    if (g_cfg_jacobi1d_ctas == 0 && g_cfg_jacobi1d_depth == 0 && tsteps >= kLeastResident) {
+      const int32_t r = jacobi1d_resident_run(a, b, n, tsteps, st);
+      if (r != NPBGB_ERR_STATE) return r;
+    }
+  }
   // H half-sweeps per launch (even) and H halo points per side; segments of w
   // points, ctas per SM, at least 32 points, and at most what keeps both
   // staged copies within the default 48 KB of dynamic shared memory (larger

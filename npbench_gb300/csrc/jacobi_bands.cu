@@ -722,29 +722,6 @@ jacobi2d_bands(T* __restrict__ A, T* __restrict__ B, int ny, int nx, int halfswe
   cluster_sync();  // shared memory stays while a band of the cluster may still send to it
 }
 
-cudaError_t scratch_pool(cudaMemPool_t* out) {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p;
-    if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
-    uint64_t keep = uint64_t(64) << 20;  // more than four calls' mail
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    pools[dev] = p;
-  }
-  *out = pools[dev];
-  return cudaSuccess;
-}
-
 // The instances: columns a thread, and the widest grid of each.
 template <typename T>
 struct Instance {
@@ -803,6 +780,30 @@ int clustered_ctas(int dev, int which, int ci, size_t smem) {
 }
 
 }  // namespace
+
+// A pool for the launches that hand values on, kept per device (also jacobi1d_resident.cu).
+cudaError_t scratch_pool(cudaMemPool_t* out) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p;
+    if ((e = cudaMemPoolCreate(&p, &props)) != cudaSuccess) return e;
+    uint64_t keep = uint64_t(64) << 20;  // more than four calls' mail
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    pools[dev] = p;
+  }
+  *out = pools[dev];
+  return cudaSuccess;
+}
 
 // Runs the whole time loop of Jacobi-2D in one cooperative launch, or returns
 // NPBGB_ERR_STATE, after which the caller uses the chained kernels: when the bands do
