@@ -132,7 +132,8 @@ def ncu_traffic(kernel_key):
 
 # Which probe measures each pipe's throughput (npbench_gb300.pipes): the integer
 # ALU pipe retires LOP3, the binary64 pipe DADD/DMUL/DFMA; the stencils' FMA-pipe
-# instructions are integer multiply-adds on its heavy half, whose rate IMAD measures.
+# instructions are packed binary32 operations and integer multiply-adds, all of them on
+# its heavy half, whose rate IMAD measures.
 PIPE_PROBES = {"alu": "lop3", "fp64": "dadd", "fma": "imad"}
 
 
@@ -414,7 +415,7 @@ def run_gb300(args, world, rank, local):
     # The arithmetic bounds.  fp64_roofline: the reference's 13 binary64
     # operations per update at the achieved rate, against what the binary64 pipe
     # alone retires (measured now by the DADD probe); above 1 because most
-    # additions run exactly in fixed point on the integer pipes.
+    # additions run exactly in binary32 limbs.
     # compute_roofline: the kernel's own instruction mix against every pipe.
     rates = measure_pipes() if rank == 0 else {}
     fp64_equiv = HEAT_FP64_OPS * INTERIOR / (launch_ms * 1e-3)

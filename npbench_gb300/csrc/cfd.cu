@@ -493,7 +493,7 @@ __device__ __forceinline__ bool collect(const ulonglong2* const (&at)[N], bool (
 }
 
 // Channel flow's verdicts.  ctl counts the steps that may change u and v.
-__device__ void channel_judge(const CfdArgs& a) {
+__device__ void channel_verdict(const CfdArgs& a) {
   double s_prev = numpy_sum_cta(a, a.u[0]);
   if (threadIdx.x == 0) st_release(a.ctl, 1u);
   for (uint32_t n = 1;; ++n) {
@@ -526,7 +526,7 @@ template <bool CH, int CPT>
 __global__ void __launch_bounds__(kCThreads)
 cfd_mail(CfdArgs a) {
   if (CH && int(blockIdx.x) == a.nbands) {
-    channel_judge(a);
+    channel_verdict(a);
     return;
   }
   extern __shared__ double field[];
@@ -908,7 +908,7 @@ int64_t round_up(int64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
 namespace {
 // The mailbox form of a grid: one band per CTA (channel flow keeps an SM for the
-// CTA that judges), a thread per one, two or four columns; bands must fit in
+// CTA that decides when to stop), a thread per one, two or four columns; bands must fit in
 // shared memory.  Larger grids take cfd_bands.
 struct MailPlan {
   bool fits = false;
@@ -916,7 +916,7 @@ struct MailPlan {
   int threads = 0, per_thread = 0;
   size_t smem = 0;
 };
-constexpr size_t kMailSmem = 190 * 1024;  // next to the judge's static 33 KB
+constexpr size_t kMailSmem = 190 * 1024;  // next to the deciding CTA's static 33 KB
 
 MailPlan mail_plan(int64_t ny, int64_t nx, bool channel) {
   MailPlan m;
@@ -926,7 +926,7 @@ MailPlan mail_plan(int64_t ny, int64_t nx, bool channel) {
   m.nb = npbgb::cdiv(ny - 2, m.rows);
   m.per_thread = nx <= npbgb::kCThreads ? 1 : nx <= 2 * npbgb::kCThreads ? 2 : 4;
   m.threads = nx <= npbgb::kCThreads ? int(npbgb::cdiv(nx, 32) * 32) : npbgb::kCThreads;
-  if (channel && m.threads < 128) m.threads = 128;  // the judge sums with them
+  if (channel && m.threads < 128) m.threads = 128;  // the deciding CTA sums with them
   m.smem = size_t(npbgb::kMailFields + (channel ? 1 : 0)) * size_t(m.rows * nx) * sizeof(double);
   m.p_bytes = round_up(m.nb * 4 * nx * int64_t(sizeof(ulonglong2)));
   m.uv_bytes = 2 * m.p_bytes;
