@@ -330,10 +330,6 @@ NPBGB_FX_FN bool within(uint32_t e) {
   return e - (static_cast<uint32_t>(135 + LO) << 23) < (static_cast<uint32_t>(HI - LO) << 23);
 }
 
-// Whether a sum had an input out of range (NaN), from its exponent fields.
-NPBGB_FX_FN bool refused(uint32_t e) { return e == 0x7f800000u; }
-NPBGB_FX_FN bool refused(P2 e) { return refused(first(e)) || refused(second(e)); }
-
 // A rounded sum of non-negative limbs, 2^-7 <= T < 8, read as T * 2^-(F - 59),
 // in binary64: the limbs' patterns next to a base are integers, their weighted
 // sum is T in units of 2^-59, and dropping the e + 7 low bits (zero after the
