@@ -35,9 +35,9 @@
 // and a point that touches one is evaluated in hardware binary64.
 //
 // Bound by the instructions of a point and by the hand-off's latency: a half-sweep of
-// binary32 1403 x 1177 takes 2.7 us where the points alone take about 1.5.  Measured,
+// binary32 1403 x 1177 takes 2.2 us where the points alone take about 1.5.  Measured,
 // chained launches to bands, TSTEPS=100: binary32 1000^2 0.72 to 0.40 ms, 1403 x 1177
-// 1.02 to 0.56, 2048^2 (TSTEPS=50) 0.785 to 0.39; binary64 300^2 (50) 0.36 to 0.25,
+// 1.02 to 0.48, 2048^2 (TSTEPS=50) 0.785 to 0.39; binary64 300^2 (50) 0.36 to 0.25,
 // 1000^2 1.68 to 1.5.  With every edge through L2 the 1403 x 1177 grid took 0.85 ms,
 // with the computing threads polling instead of extra warps 0.71.
 //
@@ -48,6 +48,7 @@
 // word, the band stops waiting, and all bands of the cluster leave together.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <mutex>
 
 #include "fxl.cuh"
@@ -448,47 +449,61 @@ __device__ __forceinline__ void run_band(T* __restrict__ A, T* __restrict__ B, i
     __syncthreads();
     const int which = !wall(0) && !near(0) ? 0 : 1;
     if (wall(which) || near(which)) return;
-    constexpr int kAtOnce = sizeof(T) == 8 ? 16 : 8, kStride = 32 * kPollWarps<T>;
-    for (int s = 1; s < halfsweeps; ++s) {
-      const typename K::Mail* from = box(which, which, uint32_t(s));
-      typename K::Halo* to = halo_at(which, s);
-      bool ok = true;
-      for (int e0 = tid - nt; e0 - lane < columns; e0 += kStride * kAtOnce) {
-        bool need[kAtOnce];
+    constexpr int kStride = 32 * kPollWarps<T>;
+    auto poll = [&](auto at_once) {
+      constexpr int kAtOnce = decltype(at_once)::value;
+      for (int s = 1; s < halfsweeps; ++s) {
+        const typename K::Mail* from = box(which, which, uint32_t(s));
+        typename K::Halo* to = halo_at(which, s);
+        bool ok = true;
+        for (int e0 = tid - nt; e0 - lane < columns; e0 += kStride * kAtOnce) {
+          bool need[kAtOnce];
 #pragma unroll
-        for (int m = 0; m < kAtOnce; ++m) need[m] = e0 + kStride * m < columns;
-        uint64_t t0 = 0;
-        for (uint32_t n = 1; ok; ++n) {
-          typename K::Letter got[kAtOnce];
+          for (int m = 0; m < kAtOnce; ++m) need[m] = e0 + kStride * m < columns;
+          uint64_t t0 = 0;
+          for (uint32_t n = 1; ok; ++n) {
+            typename K::Letter got[kAtOnce];
 #pragma unroll
-          for (int m = 0; m < kAtOnce; ++m)
-            if (need[m]) got[m] = K::peek(from + e0 + kStride * m);
-          bool missing = false;
+            for (int m = 0; m < kAtOnce; ++m)
+              if (need[m]) got[m] = K::peek(from + e0 + kStride * m);
+            bool missing = false;
 #pragma unroll
-          for (int m = 0; m < kAtOnce; ++m)
-            if (need[m]) {
-              if (K::tag(got[m]) == uint32_t(s)) {
-                to[e0 + kStride * m] = K::halo(K::cell(got[m]));
-                need[m] = false;
-              } else {
-                missing = true;
+            for (int m = 0; m < kAtOnce; ++m)
+              if (need[m]) {
+                if (K::tag(got[m]) == uint32_t(s)) {
+                  to[e0 + kStride * m] = K::halo(K::cell(got[m]));
+                  need[m] = false;
+                } else {
+                  missing = true;
+                }
               }
-            }
-          if (!missing) break;
-          if ((n & 255u) == 0) {
-            const uint64_t now = tma::globaltimer();
-            if (t0 == 0) t0 = now;
-            if (now - t0 > kJLimitNs) {
-              atomicOr(&g_jbands_error, 1u);
-              ok = false;
+            if (!missing) break;
+            if ((n & 255u) == 0) {
+              const uint64_t now = tma::globaltimer();
+              if (t0 == 0) t0 = now;
+              if (now - t0 > kJLimitNs) {
+                atomicOr(&g_jbands_error, 1u);
+                ok = false;
+              }
             }
           }
         }
+        // Field s - 2 is complete on this barrier before any warp tells it of field s.
+        if (s > 2) ok = ok && tma::mbar_wait_for(&bars[which * 2 + (s & 1)], uint32_t((s - 3) >> 1) & 1u, kJLimitNs);
+        if (!__all_sync(0xffffffffu, ok)) return;  // the computing threads' own waits run out
+        if (lane == 0) mbar_arrive(&bars[which * 2 + (s & 1)]);
       }
-      // Field s - 2 is complete on this barrier before any warp tells it of field s.
-      if (s > 2) ok = ok && tma::mbar_wait_for(&bars[which * 2 + (s & 1)], uint32_t((s - 3) >> 1) & 1u, kJLimitNs);
-      if (!__all_sync(0xffffffffu, ok)) return;  // the computing threads' own waits run out
-      if (lane == 0) mbar_arrive(&bars[which * 2 + (s & 1)]);
+    };
+    // Elements a lane asks for together: as many as it has, up to 16.  1403 x 1177 (10 a
+    // lane) takes 0.53 ms in rounds of 8, 0.485 with 16, 0.47 with 12; 1000^2 (8 a lane)
+    // 0.394 and 0.425 with 8 and 16.
+    if constexpr (sizeof(T) == 4 && CPT == 4) {
+      if (columns <= 12 * kStride)
+        poll(std::integral_constant<int, 12>{});
+      else
+        poll(std::integral_constant<int, 16>{});
+    } else {
+      poll(std::integral_constant<int, sizeof(T) == 8 ? 16 : 8>{});
     }
     return;
   }
