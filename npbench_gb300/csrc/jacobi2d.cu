@@ -97,8 +97,8 @@ jacobi2d_tma(const __grid_constant__ CUtensorMap map, const T* __restrict__ src,
 }
 
 template <int W>
-__global__ void __launch_bounds__(32 * W)
-jacobi2d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t ny, int64_t nx, int chunk) {
+__device__ __forceinline__ void limb_unit(const double* __restrict__ src, double* __restrict__ dst, int64_t ny,
+                                          int64_t nx, int chunk) {
   pdl_begin();
   const int warp = threadIdx.x >> 5;
   const int64_t k0 = 1 + (int64_t(blockIdx.x) * W + warp) * jlimb::kStrip;
@@ -108,34 +108,50 @@ jacobi2d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t 
   if (!jlimb::rows(jlimb::Limbs{fxl::consts()}, src, dst, nx, k0, ib, ie))
     jlimb::rows_hardware(src, dst, nx, k0, ib, ie);
 }
+constexpr int kLimbWarps = 4;
+// No least number of CTAs per SM here: any asked for schedules worse (5 to 8%).
+__global__ void __launch_bounds__(32 * kLimbWarps)
+jacobi2d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t ny, int64_t nx, int chunk) {
+  limb_unit<kLimbWarps>(src, dst, ny, nx, chunk);
+}
+__global__ void __launch_bounds__(32, 28)
+jacobi2d_limb_alone(const double* __restrict__ src, double* __restrict__ dst, int64_t ny, int64_t nx, int chunk) {
+  limb_unit<1>(src, dst, ny, nx, chunk);
+}
 
-// Rows per warp: an even number (two rows at a time), growing with the square root of
-// the strips' rows per warp that the GPU holds at once (36 per SM).  Measured best at
-// q = 0.1 to 2.2: 2 (600^2, TSTEPS=50: 0.425 ms, 4 0.532); 3.3: 4 (1403 x 377: 0.539,
-// 2 0.573, 6 0.652); 6.2: 6 (1000^2: 0.715, 4 0.739, 8 0.795); 15: 8 to 12 (1700 x
-// 1500); 48: 16 (2800^2); 102: 24 (4096^2).
-int limb_chunk(int64_t ny, int64_t nx) {
-  const int64_t least = cdiv(ny - 2, 65535);  // the grid's limit
-  if (g_cfg_jacobi_chunk > 0) return int(std::max<int64_t>(g_cfg_jacobi_chunk, least));
+// Warps per CTA and rows per warp, by q, the strips' rows per warp that the GPU holds at
+// once (36 per SM).  From q = 9 a warp is a CTA of its own, with 64 registers instead of
+// 56 and no neighbours to wait for at a CTA's end (1700 x 1500, TSTEPS=21: 0.530 ms
+// against 0.572; 4096^2, 5: 0.557 / 0.60; but 1000^2, 50: 0.744 / 0.711).  Rows are an
+// even number (two at a time) growing with the square root of q.  Measured best with
+// four warps at q = 0.1 to 2.2: 2 (600^2, TSTEPS=50: 0.425 ms, 4 0.532); 3.3: 4 (1403 x
+// 377: 0.539, 2 0.573, 6 0.652); 6.2: 6 (1000^2: 0.715, 4 0.739, 8 0.795); with one at
+// 15: 10 to 16; 30: 16 to 24; 48: 20 (2800^2, 11: 0.707, 10 0.736); 102: 24 to 32.
+struct LimbShape { int warps, chunk; };
+LimbShape limb_shape(int64_t ny, int64_t nx) {
   const double q = double(cdiv(nx - 2, jlimb::kStrip)) * double(ny - 2) / (36.0 * sm_count());
-  const int64_t pairs = std::max<int64_t>(int64_t(1.2 * std::sqrt(q) + 0.15), 1);
-  return int(std::max<int64_t>(2 * pairs, least + (least & 1)));
+  const bool alone = q >= 9.0;
+  const int64_t least = cdiv(ny - 2, 65535);  // the grid's limit
+  if (g_cfg_jacobi_chunk > 0) return {alone ? 1 : kLimbWarps, int(std::max<int64_t>(g_cfg_jacobi_chunk, least))};
+  const int64_t pairs = alone ? int64_t(1.5 * std::sqrt(q) + 0.5) : std::max<int64_t>(int64_t(1.2 * std::sqrt(q) + 0.15), 1);
+  return {alone ? 1 : kLimbWarps, int(std::max<int64_t>(2 * pairs, least + (least & 1)))};
 }
 
 // Binary64 in limbs (jacobi_limb.cuh).  Bound by instructions on large grids, by a
 // launch's latency on small ones.  Against the fixed-point strips and the TMA ring
 // with their best settings (ms, TSTEPS=50, 11 at 2800^2 and 4096^2; then NPBench's
 // initial field, whose values leave [0, 1)): 300^2 0.356 to 0.29 and 0.49 to 0.34;
-// 1000^2 0.84 to 0.715 and 1.31 to 0.74; 2800^2 0.95 to 0.80 and 1.80 to 0.81; 4096^2
-// 1.71 to 1.48 and 3.41 to 1.49.
+// 1000^2 0.84 to 0.715 and 1.31 to 0.74; 2800^2 0.95 to 0.71 and 1.80 to 0.72; 4096^2
+// 1.71 to 1.39 and 3.41 to 1.40.
 int32_t run_limb(double* a, double* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st) {
-  constexpr int W = 4;
-  const int chunk = limb_chunk(ny, nx);
-  const dim3 grid{unsigned(cdiv(nx - 2, W * jlimb::kStrip)), unsigned(cdiv(ny - 2, chunk))};
+  const LimbShape s = limb_shape(ny, nx);
+  const auto kern = s.warps == 1 ? jacobi2d_limb_alone : jacobi2d_limb;
+  const dim3 grid{unsigned(cdiv(nx - 2, s.warps * jlimb::kStrip)), unsigned(cdiv(ny - 2, s.chunk))};
   cudaError_t e = cudaSuccess;
   for (int32_t t = 1; t < tsteps && e == cudaSuccess; ++t) {
-    e = launch_chained(jacobi2d_limb<W>, grid, dim3{32u * W}, 0, st, a, b, ny, nx, chunk);
-    if (e == cudaSuccess) e = launch_chained(jacobi2d_limb<W>, grid, dim3{32u * W}, 0, st, b, a, ny, nx, chunk);
+    e = launch_chained(kern, grid, dim3{32u * unsigned(s.warps)}, 0, st, static_cast<const double*>(a), b, ny, nx, s.chunk);
+    if (e == cudaSuccess)
+      e = launch_chained(kern, grid, dim3{32u * unsigned(s.warps)}, 0, st, static_cast<const double*>(b), a, ny, nx, s.chunk);
   }
   return cuda_status(e, "jacobi2d_limb");
 }

@@ -136,3 +136,26 @@ def test_jacobi_limbs_at_strip_edges(shape, values):
     finally:
         for k, v in old:
             _lib.set_config(k, v)
+
+
+# Large grids, whose warps are CTAs of their own: an odd number of rows and of strips, the
+# last strip of one column.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1301, 1263), (4003, 453)])
+@pytest.mark.parametrize("values", ["unit", "npbench", "signed"])
+def test_jacobi_limbs_on_large_grids(shape, values):
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from conftest import bits_equal
+    from npbench_gb300 import stencils
+    from oracle import cref
+    rng = np.random.default_rng(9)
+    i, j = np.indices(shape)
+    A = (rng.random(shape) if values == "unit" else rng.standard_normal(shape) if values == "signed"
+         else i * (j + 2) / shape[0])
+    B = A[::-1].copy()
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    stencils.jacobi_2d_kernel(3, dA, dB)
+    cref.jacobi_2d_kernel(3, A, B)
+    assert bits_equal(dA.cpu().numpy(), A) and bits_equal(dB.cpu().numpy(), B)
