@@ -48,11 +48,13 @@ __device__ __forceinline__ double eighth_of(double w) {
 __device__ __forceinline__ double neg(double x) {
   return __longlong_as_double(__double_as_longlong(x) ^ static_cast<long long>(0x8000000000000000ull));
 }
-// q_k * (u[k-1] - u[k]) from level k-1's product q_k * (u[k] - u[k-1]): rounding is
-// symmetric, so it is the product negated, the signs of zeros included, but for equal
+// q_k * (u[k-1] - u[k]).  REUSE: from level k-1's product q_k * (u[k] - u[k-1]); rounding
+// is symmetric, so it is the product negated, the signs of zeros included, but for equal
 // values, whose difference is +0 both ways (or NaN).  Two of the about 26 binary64
 // operations of a level less: 256 x 256 x 160 takes 574 us instead of 606.
-__device__ __forceinline__ double from_below(double product, double below, double here) {
+template <bool REUSE>
+__device__ __forceinline__ double from_below(double q, double product, double below, double here) {
+  if constexpr (!REUSE) return mul_rn(q, sub_rn(below, here));
   return __double_as_longlong(below) == __double_as_longlong(here) ? product : neg(product);
 }
 __device__ __forceinline__ double ld(const double* p) { return __ldg(p); }
@@ -98,8 +100,8 @@ vadv_columns(double* __restrict__ us, const double* __restrict__ u, const double
   // k = 0 (slots 0 and 1)
   double qn = eighth_of(add_rn(r[1].wh, r[1].wl));  // q_1
   double ucur = r[0].u, unext = r[1].u;
-  double qdu = mul_rn(qn, sub_rn(unext, ucur));  // q_{k+1} * (u[k+1] - u[k])
-  double d = add_rn(add_rn(add_rn(mul_rn(dtr, r[0].up), r[0].ut), r[0].s), neg(qdu));
+  double d = add_rn(add_rn(add_rn(mul_rn(dtr, r[0].up), r[0].ut), r[0].s),
+                    mul_rn(neg(qn), sub_rn(unext, ucur)));
   double dv = __drcp_rn(sub_rn(dtr, qn));
   double cprev = mul_rn(qn, dv);
   double dprev = mul_rn(d, dv);
@@ -117,12 +119,11 @@ vadv_columns(double* __restrict__ us, const double* __restrict__ u, const double
       const FwdLevel& nxt = r[(j + 1) % kRing];
       const double q = qn;                                 // -acol = -as
       qn = eighth_of(add_rn(nxt.wh, nxt.wl));              // cs = unscaled ccol_k
-      const double first = from_below(qdu, ucur, unext);
+      const double uprev = ucur;
       ucur = unext;
       unext = nxt.u;
-      qdu = mul_rn(qn, sub_rn(unext, ucur));
       const double acol = neg(q);
-      const double corr = sub_rn(first, qdu);
+      const double corr = sub_rn(mul_rn(q, sub_rn(uprev, ucur)), mul_rn(qn, sub_rn(unext, ucur)));
       d = add_rn(add_rn(add_rn(mul_rn(dtr, cur.up), cur.ut), cur.s), corr);
       const double bcol = sub_rn(sub_rn(dtr, acol), qn);
       dv = __drcp_rn(sub_rn(bcol, mul_rn(cprev, acol)));
@@ -140,7 +141,7 @@ vadv_columns(double* __restrict__ us, const double* __restrict__ u, const double
   {
     const double q = qn;
     const double acol = neg(q);
-    const double corr = from_below(qdu, ucur, unext);  // (-as)*(u[K-2] - u[K-1])
+    const double corr = mul_rn(q, sub_rn(ucur, unext));    // (-as)*(u[K-2] - u[K-1])
     d = add_rn(add_rn(add_rn(mul_rn(dtr, last.up), last.ut), last.s), corr);
     const double bcol = sub_rn(dtr, acol);
     dv = __drcp_rn(sub_rn(bcol, mul_rn(cprev, acol)));
@@ -202,6 +203,7 @@ __device__ __forceinline__ void st4(double* p, const double (&v)[4]) {
 
 // 7 CTAs of 64 threads per SM (at most 144 registers a thread) keep the
 // 256x256-column paper problem (6.7 CTAs per SM) in a single wave.
+template <bool REUSE>
 __global__ void __launch_bounds__(kThreads, 7)
 vadv_columns_v4(double* __restrict__ us, const double* __restrict__ u,
                 const double* __restrict__ wcon, const double* __restrict__ up,
@@ -247,7 +249,7 @@ vadv_columns_v4(double* __restrict__ us, const double* __restrict__ u,
       } else if (k < K - 1) {
         const double q = qn;
         qn = eighth_of(add_rn(wh1, wl1));
-        const double first = from_below(qdu, ucur, unext);
+        const double first = from_below<REUSE>(q, qdu, ucur, unext);
         ucur = unext;
         unext = u1;
         qdu = mul_rn(qn, sub_rn(unext, ucur));
@@ -263,7 +265,7 @@ vadv_columns_v4(double* __restrict__ us, const double* __restrict__ u,
       } else {
         const double q = qn;
         const double acol = neg(q);
-        const double corr = from_below(qdu, ucur, unext);  // (-as)*(u[K-2] - u[K-1])
+        const double corr = from_below<REUSE>(q, qdu, ucur, unext);  // (-as)*(u[K-2] - u[K-1])
         const double d =
             add_rn(add_rn(add_rn(mul_rn(dtr, cur.up[j]), cur.ut[j]), cur.s[j]), corr);
         const double bcol = sub_rn(dtr, acol);
@@ -371,16 +373,16 @@ extern "C" int32_t npbgb_vadv(void* utens_stage, const void* u_stage, const void
   auto a32 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; };
   const bool sector = K % 4 == 0 && a32(utens_stage) && a32(u_stage) && a32(wcon) &&
                       a32(u_pos) && a32(utens);
-  if (sector)
-    vadv_columns_v4<<<unsigned(blocks), kThreads, 0, st>>>(
-        static_cast<double*>(utens_stage), static_cast<const double*>(u_stage),
-        static_cast<const double*>(wcon), static_cast<const double*>(u_pos),
-        static_cast<const double*>(utens), dtr_stage, ncol, J, K, static_cast<double*>(ws));
-  else
-    vadv_columns<<<unsigned(blocks), kThreads, 0, st>>>(
-        static_cast<double*>(utens_stage), static_cast<const double*>(u_stage),
-        static_cast<const double*>(wcon), static_cast<const double*>(u_pos),
-        static_cast<const double*>(utens), dtr_stage, ncol, J, K, static_cast<double*>(ws));
+  // The products handed on from two CTAs per SM up, where the binary64 pipe binds; with
+  // fewer a level's chain does, and they lengthen it (K = 40 / 160: 106 x 144 columns 80.0
+  // / 217 us without, 80.7 / 220 with; 128 x 160 97.8 / 285 and 95.4 / 277).
+  const auto kern = !sector                  ? vadv_columns
+                    : blocks > 2 * sm_count() ? vadv_columns_v4<true>
+                                              : vadv_columns_v4<false>;
+  kern<<<unsigned(blocks), kThreads, 0, st>>>(
+      static_cast<double*>(utens_stage), static_cast<const double*>(u_stage),
+      static_cast<const double*>(wcon), static_cast<const double*>(u_pos),
+      static_cast<const double*>(utens), dtr_stage, ncol, J, K, static_cast<double*>(ws));
   cudaError_t le = counted(cudaGetLastError());
   if (workspace == nullptr) cudaFreeAsync(ws, st);
   return cuda_status(le, "vadv_columns");

@@ -1,4 +1,4 @@
-"""Vertical advection where neighbouring levels of u are equal, opposite zeros, infinite or
+"""Vertical advection (few columns and many) where neighbouring levels of u are equal, opposite zeros, infinite or
 NaN: the product that one level hands to the next, against the oracle."""
 import numpy as np
 import pytest
@@ -8,7 +8,7 @@ from oracle import cref
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", [(3, 5, 2), (4, 3, 3), (3, 4, 8), (5, 7, 13), (2, 33, 40)])
+@pytest.mark.parametrize("shape", [(3, 5, 2), (4, 3, 3), (3, 4, 8), (5, 7, 13), (2, 33, 40), (139, 141, 4), (140, 141, 8)])
 @pytest.mark.parametrize("values", ["few", "zeros", "special"])
 def test_products_handed_on(shape, values):
     import torch
