@@ -218,6 +218,12 @@ NPBGB_API int32_t npbgb_device_status(void* stream);
  * no fault.  No counterpart in the reference. */
 NPBGB_API int32_t npbgb_selftest_wait_timeout(int64_t limit_ns, void* stream);
 
+/* How the calling thread's next cooperative launch is made: 0 as always,
+ * NPBGB_LAUNCH_UNCLUSTERED without its cluster dimension, as Nsight Compute
+ * makes it.  The results must not differ.  No counterpart in the reference. */
+#define NPBGB_LAUNCH_UNCLUSTERED 1
+NPBGB_API int32_t npbgb_selftest_launch(int32_t how);
+
 /* Converts n elements: NPBGB_F32 -> NPBGB_F64 (exact) or NPBGB_F64 -> NPBGB_F32
  * (round to nearest even, as NumPy's astype).  For binary32 requests that run
  * in binary64 because their binary32 error would exceed NPBench's acceptance

@@ -45,6 +45,7 @@ NPBGB_CFG_JACOBI_FX_MUL = 24
 NPBGB_CFG_JACOBI_FX_ADDS = 25
 NPBGB_CFG_JACOBI_TMA = 26
 NPBGB_CFG_BATCH_TMA = 27
+NPBGB_LAUNCH_UNCLUSTERED = 1
 NPBGB_BATCH_PERSISTENT = 1
 NPBGB_BATCH_STEPPED = 2
 NPBGB_BATCH_QUEUE = 3
@@ -72,6 +73,7 @@ SIGNATURES = {
     "npbgb_get_config": (_i32, [_i32, ctypes.POINTER(_i64)]),
     "npbgb_device_status": (_i32, [_vp]),
     "npbgb_selftest_wait_timeout": (_i32, [_i64, _vp]),
+    "npbgb_selftest_launch": (_i32, [_i32]),
     "npbgb_batch_create": (_i32, [ctypes.POINTER(Grid), _i64, _i32, ctypes.POINTER(_vp)]),
     "npbgb_batch_launch": (_i32, [_vp, _i32, _vp]),
     "npbgb_batch_replan": (_i32, [_vp, ctypes.POINTER(Grid), _i64, _i32]),

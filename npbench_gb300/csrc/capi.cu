@@ -64,6 +64,23 @@ int32_t set_error(int32_t code, const char* fmt, ...) {
   return code;
 }
 
+// What npbgb_selftest_launch asked for, for the calling thread's next cooperative launch.
+static thread_local int32_t g_next_launch = 0;
+
+cudaError_t launch_together(const cudaLaunchConfig_t& cfg, const void* kernel, void** args) {
+  const int32_t how = g_next_launch;
+  g_next_launch = 0;
+  cudaLaunchAttribute attr[4];
+  cudaLaunchConfig_t c = cfg;
+  if (how == NPBGB_LAUNCH_UNCLUSTERED) {
+    c.attrs = attr;
+    c.numAttrs = 0;
+    for (unsigned n = 0; n < cfg.numAttrs; ++n)
+      if (cfg.attrs[n].id != cudaLaunchAttributeClusterDimension) attr[c.numAttrs++] = cfg.attrs[n];
+  }
+  return counted(cudaLaunchKernelExC(&c, kernel, args));
+}
+
 namespace tma {
 
 static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -300,6 +317,13 @@ int32_t npbgb_selftest_wait_timeout(int64_t limit_ns, void* stream) {
   using namespace npbgb;
   if (limit_ns <= 0 || limit_ns > 2000000000) return set_error(NPBGB_ERR_ARG, "limit out of range");
   return launch_wait_timeout_selftest(uint64_t(limit_ns), as_stream(stream));
+}
+
+int32_t npbgb_selftest_launch(int32_t how) {
+  using namespace npbgb;
+  if (how != 0 && how != NPBGB_LAUNCH_UNCLUSTERED) return set_error(NPBGB_ERR_ARG, "unknown kind of launch %d", how);
+  g_next_launch = how;
+  return NPBGB_OK;
 }
 
 }  // extern "C"

@@ -46,6 +46,10 @@
 // whose thread sent it after it had taken s-1; so the place of s-1 is free by then.
 // Every wait is bounded: a neighbour that sends nothing for seconds sets an error
 // word, the band stops waiting, and all bands of the cluster leave together.
+//
+// Mail and halos are laid out for the cluster size that the host asked for.  A launch
+// that runs in other clusters (Nsight Compute launches a cooperative kernel's CTAs one
+// by one) is told by the hardware's own count and takes in_memory instead.
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -726,10 +730,58 @@ __device__ __forceinline__ void run_band(T* __restrict__ A, T* __restrict__ B, i
   dump(A);
 }
 
+// The same half-sweeps in global memory, for a launch without its clusters: rows dealt
+// out to `parts` CTAs (all resident, as the launch is cooperative), which meet after
+// every half-sweep at `arrived`.
+template <typename T>
+__device__ __noinline__ void in_memory(T* A, T* B, int ny, int nx, int halfsweeps, int parts, uint32_t* arrived) {
+  if (int(blockIdx.x) >= parts) return;
+  for (int s = 0; s < halfsweeps; ++s) {
+    const T* src = s & 1 ? B : A;
+    T* dst = s & 1 ? A : B;
+    for (int i = 1 + int(blockIdx.x); i < ny - 1; i += parts)
+      for (int j = 1 + int(threadIdx.x); j < nx - 1; j += int(blockDim.x)) {
+        const int64_t at = int64_t(i) * nx + j;
+        const T* p = src + at;
+        T sum = add_rn(__ldcg(p), __ldcg(p - 1));
+        sum = add_rn(sum, __ldcg(p + 1));
+        sum = add_rn(sum, __ldcg(p + nx));
+        sum = add_rn(sum, __ldcg(p - nx));
+        __stcg(dst + at, mul_rn(T(0.2), sum));
+      }
+    __syncthreads();
+    if (parts == 1) continue;
+    bool ok = true;
+    if (threadIdx.x == 0) {
+      const uint32_t all = uint32_t(parts) * uint32_t(s + 1);
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+      const uint64_t t0 = tma::globaltimer();
+      for (;;) {
+        uint32_t v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+        if (int32_t(v - all) >= 0) break;
+        if (tma::globaltimer() - t0 > kJLimitNs) {
+          atomicOr(&g_jbands_error, 1u);
+          ok = false;
+          break;
+        }
+      }
+    }
+    if (__syncthreads_or(!ok)) return;
+  }
+}
+
+// in_cluster: the CTAs of a cluster that base, extra and mail are meant for.
 template <typename T, int CPT>
 __global__ void __launch_bounds__(kCompute<T, CPT> + 32 * kPollWarps<T>, 1)
 jacobi2d_bands(T* __restrict__ A, T* __restrict__ B, int ny, int nx, int halfsweeps, int base, int extra, int nb,
-               typename Kind<T>::Mail* __restrict__ mail) {
+               int in_cluster, typename Kind<T>::Mail* __restrict__ mail, uint32_t* __restrict__ arrived) {
+  uint32_t size;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+  if (int(size) != in_cluster) {  // the same for every CTA of the launch
+    in_memory<T>(A, B, ny, nx, halfsweeps, int(gridDim.x) > in_cluster ? nb : 1, arrived);
+    return;
+  }
   if (int(blockIdx.x) < nb)
     run_band<T, CPT>(A, B, ny, nx, halfsweeps, base, extra, nb, mail);
   else
@@ -740,7 +792,7 @@ jacobi2d_bands(T* __restrict__ A, T* __restrict__ B, int ny, int nx, int halfswe
 // The instances: columns a thread, and the widest grid of each.
 template <typename T>
 struct Instance {
-  using Kernel = void (*)(T*, T*, int, int, int, int, int, int, typename Kind<T>::Mail*);
+  using Kernel = void (*)(T*, T*, int, int, int, int, int, int, int, typename Kind<T>::Mail*, uint32_t*);
   Kernel kern;
   int cpt, compute;
   size_t (*bytes)(int H, int threads);
@@ -871,7 +923,8 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   const bool wide = sizeof(T) == 4 && which == 2;
   if (!any && (tsteps < (wide ? 16 : 8) || (sizeof(T) == 8 && H > 2) || (wide && H < 3))) return NPBGB_ERR_STATE;
   const int nb = int(cdiv(interior, 2 * H)), clusters = int(cdiv(nb, in_cluster));
-  const size_t bytes = size_t(4) * clusters * size_t(columns) * sizeof(typename Kind<T>::Mail);
+  const size_t mail_bytes = size_t(4) * clusters * size_t(columns) * sizeof(typename Kind<T>::Mail);
+  const size_t bytes = mail_bytes + 256;  // and a counter
   cudaMemPool_t pool;
   void* scratch = nullptr;
   cudaError_t e;
@@ -883,9 +936,10 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   if (clusters > 1) e = cudaMemsetAsync(scratch, 0, bytes, st);
   if (e == cudaSuccess) {
     auto* mail = static_cast<typename Kind<T>::Mail*>(scratch);
+    auto* arrived = reinterpret_cast<uint32_t*>(static_cast<unsigned char*>(scratch) + mail_bytes);
     int ny_ = int(ny), nx_ = int(nx), hs = 2 * (tsteps - 1), nb_ = nb;
     int base = int(interior / nb), extra = int(interior % nb);
-    void* args[] = {&a, &b, &ny_, &nx_, &hs, &base, &extra, &nb_, &mail};
+    void* args[] = {&a, &b, &ny_, &nx_, &hs, &base, &extra, &nb_, &in_cluster, &mail, &arrived};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(clusters * in_cluster));
     cfg.blockDim = dim3(unsigned(compute + 32 * kPollWarps<T>));
@@ -899,7 +953,7 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    e = counted(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(in.kern), args));
+    e = launch_together(cfg, reinterpret_cast<const void*>(in.kern), args);
   }
   cudaFreeAsync(scratch, st);
   return cuda_status(e, "jacobi2d_bands");

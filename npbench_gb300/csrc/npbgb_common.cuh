@@ -105,6 +105,10 @@ inline cudaError_t counted(cudaError_t e) {
   if (e == cudaSuccess) add_launches(1);
   return e;
 }
+
+// A counted cooperative launch (npbgb_selftest_launch can change the next one).
+cudaError_t launch_together(const cudaLaunchConfig_t& cfg, const void* kernel, void** args);
+
 extern int64_t g_cfg_hdiff_emu;  // NPBGB_CFG_HDIFF_EMU
 
 // allow_pdl = false launches in plain stream order whatever NPBGB_CFG_PDL says
