@@ -495,6 +495,7 @@ __device__ __forceinline__ void run_band(T* __restrict__ A, T* __restrict__ B, i
         // Field s - 2 is complete on this barrier before any warp tells it of field s.
         if (s > 2) ok = ok && tma::mbar_wait_for(&bars[which * 2 + (s & 1)], uint32_t((s - 3) >> 1) & 1u, kJLimitNs);
         if (!__all_sync(0xffffffffu, ok)) return;  // the computing threads' own waits run out
+        __syncwarp();  // orders every lane's cells before lane 0's arrival; a vote does not
         if (lane == 0) mbar_arrive(&bars[which * 2 + (s & 1)]);
       }
     };
