@@ -665,7 +665,8 @@ __device__ __forceinline__ void run_band(T* __restrict__ A, T* __restrict__ B, i
       }
 #pragma unroll 1
       for (int p = 0; p < H; ++p) {
-        if (p == seconds - 1 || (p == 0 && seconds == 0)) place_below(s);
+        const bool at_below = p == seconds - 1 || (p == 0 && seconds == 0);
+        if (at_below) place_below(s);
 #pragma unroll
         for (int c = 0; c < CPT; ++c) at[c] += lay.row;
         if (p + 1 < H) {
@@ -674,7 +675,9 @@ __device__ __forceinline__ void run_band(T* __restrict__ A, T* __restrict__ B, i
         } else {
 #pragma unroll
           for (int c = 0; c < CPT; ++c) {
-            const Cell below = halo_cell(1, s, c);
+            // Without a second row here that half is not used, and the halo's place may
+            // already be the neighbour's again: the last second row has been sent.
+            const Cell below = at_below ? halo_cell(1, s, c) : K::half(cur[c], 1);
             south[c] = K::join(seconds == 0 ? below : row_h[c], below);
           }
         }
