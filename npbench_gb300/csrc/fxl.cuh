@@ -291,11 +291,15 @@ NPBGB_FX_FN uint32_t frame_of(uint32_t top) {
   return keep ? 0u : static_cast<uint32_t>(e + 1) << 20;
 }
 
-// Whether from_f64 refused either value.
+// Whether from_f64 refuses the binary64 x.
+NPBGB_FX_FN bool refused(const Consts& k, uint64_t x) {
+  return static_cast<uint32_t>(x >> 32) - k.scale - 0x3f800000u >= 0x700000u && x != 0;
+}
+// Whether it refused either value.
 NPBGB_FX_FN bool refused_value(const L3& x) {
   return (first(x.h) << 1) > 0xff000000u || (second(x.h) << 1) > 0xff000000u;
 }
-// Whether it refused both.
+// Whether it refused both values.
 NPBGB_FX_FN bool refused_both(const L3& x) {
   return (first(x.h) << 1) > 0xff000000u && (second(x.h) << 1) > 0xff000000u;
 }

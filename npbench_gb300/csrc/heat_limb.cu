@@ -91,13 +91,73 @@ __device__ __noinline__ double other_point(const double* q, int64_t s0, int64_t 
   return hcore::heat_point<double>(q[0], q[s0], q[-s0], q[s1], q[-s1], q[1], q[-1]);
 }
 
-// A CTA's tile and chunk.  SCALED: in the frame that the values at the corners of its
-// first plane (the same for every thread) ask for.  Otherwise in the frame of zero,
-// which costs no instructions, and false (nothing written) if a centre pair of the
-// first plane is out of range.
+// A CTA's tile and chunk in hardware binary64.  The tile's columns are numbered along its
+// rows, so that one which the array cuts short fills its warps all the same; a thread
+// streams one in every 32 W of them, with in-plane neighbours from memory.  Bound by the
+// binary64 pipe, nine operations a point, and the last wave of CTAs: standard normal
+// values at 256^3, TSTEPS=11, 6.1 ms (the pipe alone 5.86), where limbs evaluated in
+// vain first and points one by one took 6.8; two of the nine on the integer pipes
+// (f64emu.cuh) 6.6.
+template <int W, int R>
+__device__ __noinline__ void run_hardware(const double* __restrict__ src, double* __restrict__ dst, int64_t n0,
+                                          int64_t n1, int64_t n2, int chunk) {
+  constexpr int kEach = 2 * R;
+  const int64_t k0 = 1 + int64_t(blockIdx.x) * 32, j0 = 1 + int64_t(blockIdx.y) * Geom<W, R>::kTileRows;
+  const int ib = 1 + int(blockIdx.z) * chunk;
+  const int ie = ib + chunk < int(n0) - 1 ? ib + chunk : int(n0) - 1;
+  const int columns = int(n2 - 1 - k0 < 32 ? n2 - 1 - k0 : 32);
+  const int rows = int(n1 - 1 - j0 < Geom<W, R>::kTileRows ? n1 - 1 - j0 : Geom<W, R>::kTileRows);
+  const int64_t s0 = n1 * n2;
+  const double* p = src + int64_t(ib) * s0 + j0 * n2 + k0;
+  double* o = dst + (p - src);
+  const int first = int(threadIdx.x) & ~31;  // of the warp's columns
+  const int points = rows * columns;
+  uint32_t off[kEach];
+  bool live[kEach];
+  double before[kEach], at[kEach];
+#pragma unroll
+  for (int m = 0; m < kEach; ++m) {
+    const int q = int(threadIdx.x) + m * 32 * W;
+    live[m] = q < points;
+    off[m] = live[m] ? uint32_t(q / columns) * uint32_t(n2) + uint32_t(q % columns) : 0u;
+    before[m] = p[int64_t(off[m]) - s0];
+    at[m] = p[off[m]];
+  }
+  for (int i = ib; i < ie; ++i) {
+    double after[kEach], jp[kEach], jm[kEach], kp[kEach], km[kEach];
+#pragma unroll
+    for (int m = 0; m < kEach; ++m)
+      if (first + m * 32 * W < points) {
+        const double* c = p + off[m];
+        after[m] = c[s0];
+        jp[m] = c[n2];
+        jm[m] = c[-n2];
+        kp[m] = c[1];
+        km[m] = c[-1];
+      }
+#pragma unroll
+    for (int m = 0; m < kEach; ++m)
+      if (first + m * 32 * W < points) {
+        const double v = hcore::heat_point<double>(at[m], after[m], before[m], jp[m], jm[m], kp[m], km[m]);
+        if (live[m]) o[off[m]] = v;
+        before[m] = at[m];
+        at[m] = after[m];
+      }
+    p += s0;
+    o += s0;
+  }
+}
+
+// A CTA's tile and chunk; 0 when it is done.  SCALED: in the frame that the values at the
+// corners of its first plane (the same for every thread) ask for; with R = 2, not 0
+// (nothing written) if three of four rows of pairs of that plane hold a value out of the
+// frame, as nearly every warp would then evaluate its points twice.  Otherwise in the
+// frame of zero, which costs no instructions, and not 0 (nothing written) if a centre
+// pair of the first plane is out of range: bit 2 + r then says that one of the thread's
+// pair r is negative.
 template <int W, int R, bool SCALED>
-__device__ __forceinline__ bool run_chunk(const double* __restrict__ src, double* __restrict__ dst, int64_t n0,
-                                          int64_t n1, int64_t n2, int chunk, Plane<W, R> (&plane)[3]) {
+__device__ __forceinline__ int run_chunk(const double* __restrict__ src, double* __restrict__ dst, int64_t n0,
+                                         int64_t n1, int64_t n2, int chunk, Plane<W, R> (&plane)[3]) {
   using G = Geom<W, R>;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t k0 = 1 + int64_t(blockIdx.x) * 32, j0 = 1 + int64_t(blockIdx.y) * G::kTileRows;
@@ -178,11 +238,22 @@ __device__ __forceinline__ bool run_chunk(const double* __restrict__ src, double
     for (int c = 0; c < 4; ++c) top = corner[c] < 0x7ff00000u && corner[c] > top ? corner[c] : top;
     K.scale = fxl::frame_of(top);
   }
+  if (SCALED && R == 2) {
+    bool counts = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const bool a = in_a[r] && fxl::refused(K, bits_of(own1[r].a)), b = in_b[r] && fxl::refused(K, bits_of(own1[r].b));
+      if (__any_sync(0xffffffffu, a || b) && tx == r) counts = true;
+    }
+    if (__syncthreads_count(counts) * 4 >= 3 * W * R) return 1;
+  }
 #pragma unroll
   for (int r = 0; r < R; ++r) x0[r] = limbs(own[r]);
   bool out_of_range = false;
+  uint32_t negative = 0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
+    if (!SCALED && int((bits_of(own1[r].a) | bits_of(own1[r].b)) >> 32) < 0) negative |= 4u << r;
     x1[r] = limbs(own1[r]);
     out_of_range = out_of_range || fxl::refused_both(x1[r]);
     plane[0].put(row + r + 1, tx + 1, x1[r]);
@@ -194,7 +265,7 @@ __device__ __forceinline__ bool run_chunk(const double* __restrict__ src, double
   if (SCALED)
     __syncthreads();
   else if (__syncthreads_or(out_of_range))
-    return false;
+    return int(1u | negative);
 
   double* o = dst + int64_t(ib) * s0;
   int i = ib;
@@ -247,29 +318,39 @@ __device__ __forceinline__ bool run_chunk(const double* __restrict__ src, double
   // The register sets and buffers change roles by unrolling, without moves.
   while (step(x0, x1, x2, 0) && step(x1, x2, x0, 1) && step(x2, x0, x1, 2)) {
   }
-  return true;
+  return 0;
 }
 
-// Out of line, so that the kernel's registers are the other form's.
+// Out of line, so that the kernel's registers are the other form's.  Bit r of `negative`:
+// one of the thread's pair r is negative, which no frame holds.
 template <int W, int R>
 __device__ __noinline__ void run_scaled(const double* __restrict__ src, double* __restrict__ dst, int64_t n0,
-                                        int64_t n1, int64_t n2, int chunk, Plane<W, R> (&plane)[3]) {
-  run_chunk<W, R, true>(src, dst, n0, n1, n2, chunk, plane);
+                                        int64_t n1, int64_t n2, int chunk, uint32_t negative,
+                                        Plane<W, R> (&plane)[3]) {
+  bool counts = false;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (__any_sync(0xffffffffu, (negative >> r) & 1u) && int(threadIdx.x & 31) == r) counts = true;
+  if (__syncthreads_count(counts) * 4 >= 3 * W * R || run_chunk<W, R, true>(src, dst, n0, n1, n2, chunk, plane))
+    run_hardware<W, R>(src, dst, n0, n1, n2, chunk);
 }
 
 // With two pairs a thread a CTA tries the frame of zero first: the scale in every
 // conversion costs 3.5% at 256^3.  With one pair that form needs more registers than
-// seven CTAs per SM leave (120^3: 0.605 ms against 0.593, and 0.58 without any scale).
+// seven CTAs per SM leave (120^3: 0.605 ms against 0.593, and 0.58 without any scale), and
+// so does run_hardware (130^3, TSTEPS=21: 0.733 ms against 0.707, for 1.68 against 1.71
+// on standard normal values).
 template <int W, int R>
 __global__ void __launch_bounds__(32 * W, kCtas<R>)
 heat3d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t n0, int64_t n1,
             int64_t n2, int chunk) {
   pdl_begin();
   __shared__ Plane<W, R> plane[3];
-  if constexpr (R == 1)
+  if constexpr (R == 1) {
     run_chunk<W, R, true>(src, dst, n0, n1, n2, chunk, plane);
-  else if (!run_chunk<W, R, false>(src, dst, n0, n1, n2, chunk, plane))
-    run_scaled<W, R>(src, dst, n0, n1, n2, chunk, plane);
+  } else if (const int how = run_chunk<W, R, false>(src, dst, n0, n1, n2, chunk, plane)) {
+    run_scaled<W, R>(src, dst, n0, n1, n2, chunk, uint32_t(how) >> 2, plane);
+  }
 }
 
 template <int R>
