@@ -427,16 +427,13 @@ NPBGB_FX_FN double mul02_wide(int64_t w) {
   return w == 0 ? 0.0 : double_of(bits);
 }
 
-// RN(0.2 * x) for a binary64 x, on the integer pipes when x is normal with a
-// biased exponent in [24, 2000] (then the product is normal too): the 53-bit
-// significand times M (106 bits) rounded once to nearest even, as mul02 does;
-// any other x (zeros, subnormals, huge, infinite, NaN) takes the hardware
-// multiply.
-NPBGB_FX_FN double mul02_any(double x) {
+// RN(0.2 * x) for a binary64 x that is normal with a biased exponent in [24, 2000] (then
+// the product is normal too), on the integer pipes: the 53-bit significand times M (106
+// bits) rounded once to nearest even, as mul02 does.
+NPBGB_FX_FN double mul02_normal(double x) {
   constexpr uint64_t M = 0x1999999999999Aull;
   const uint64_t b = bits_of(x);
   const uint32_t e = static_cast<uint32_t>(b >> 52) & 0x7ffu;
-  if (e - 24u > 2000u - 24u) return 0.2 * x;
   const uint64_t sig = (b & 0xfffffffffffffull) | 0x10000000000000ull;
 #if defined(__CUDA_ARCH__)
   const uint64_t lo = sig * M;
@@ -456,6 +453,11 @@ NPBGB_FX_FN double mul02_any(double x) {
                        (s - (uint64_t(1) << 52));
   return double_of(mag | (b & 0x8000000000000000ull));
 }
+NPBGB_FX_FN bool mul02_is_normal(double x) {
+  return (static_cast<uint32_t>(bits_of(x) >> 52) & 0x7ffu) - 24u <= 2000u - 24u;
+}
+// Any other x (zeros, subnormals, huge, infinite, NaN) takes the hardware multiply.
+NPBGB_FX_FN double mul02_any(double x) { return mul02_is_normal(x) ? mul02_normal(x) : 0.2 * x; }
 
 }  // namespace fx
 }  // namespace npbgb
