@@ -106,9 +106,10 @@ extern "C" {
 #define NPBGB_CFG_JACOBI_BANDS 18     /* jacobi2d: the whole time loop in one launch with
                                          bands of rows resident in shared memory.
                                          1 (default): where they measured faster
-                                         (binary32 that fits, small binary64 grids);
-                                         2: whenever the bands fit; 0: chained
-                                         launches.  Results are identical either way. */
+                                         (binary32 that fits; small binary64 grids run
+                                         in one launch over global memory); 2: whenever
+                                         the bands fit; 0: chained launches.  Results
+                                         are identical either way. */
 #define NPBGB_CFG_JACOBI_BANDS_WARPS 19 /* 8, 16, 32 or 0 (default); kept for callers
                                            that set it: the bands' threads follow from
                                            the grid's width */

@@ -33,6 +33,9 @@ extern int64_t g_cfg_jacobi_hw_warps;
 extern int64_t g_cfg_jacobi_fx_mul;
 extern int64_t g_cfg_jacobi_fx_adds;
 extern int64_t g_cfg_jacobi_tma;
+extern int64_t g_cfg_jacobi_bands;
+
+cudaError_t scratch_pool(cudaMemPool_t* out);  // jacobi_bands.cu
 
 template <typename T>
 int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st);
@@ -63,7 +66,7 @@ jacobi2d_strip(const T* __restrict__ src, T* __restrict__ dst, int64_t ny, int64
     jcore::strip_rows<T, FX, false, FX ? 1 : kUnroll, MAD, IMUL>(src, dst, nx, k0, ib, ie, one);
 }
 
-__device__ unsigned int g_jacobi_tma_error;  // bit 0: an mbarrier wait timed out
+__device__ unsigned int g_jacobi_tma_error;  // a wait gave up; bit 0: on an mbarrier, 1: on a neighbouring CTA
 
 using jcore::kTmaRing;
 using jcore::kTmaRows;
@@ -109,6 +112,8 @@ __device__ __forceinline__ void limb_unit(const double* __restrict__ src, double
     jlimb::rows_hardware(src, dst, nx, k0, ib, ie);
 }
 constexpr int kLimbWarps = 4;
+constexpr int kLoopWarps = 25;
+constexpr uint64_t kLoopLimitNs = 2000000000ull;
 // No least number of CTAs per SM here: any asked for schedules worse (5 to 8%).
 __global__ void __launch_bounds__(32 * kLimbWarps)
 jacobi2d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t ny, int64_t nx, int chunk) {
@@ -117,6 +122,51 @@ jacobi2d_limb(const double* __restrict__ src, double* __restrict__ dst, int64_t 
 __global__ void __launch_bounds__(32, 28)
 jacobi2d_limb_alone(const double* __restrict__ src, double* __restrict__ dst, int64_t ny, int64_t nx, int chunk) {
   limb_unit<1>(src, dst, ny, nx, chunk);
+}
+
+// The whole time loop in one cooperative launch, for small grids: a warp keeps one unit (a
+// strip by `chunk` rows, numbered along the rows of strips).  Half-sweep s starts when
+// the CTAs with a unit next to one of this CTA's, at most `near` away, have done s of
+// them: they then have written what it reads and read what it writes.  Bound by that
+// hand-off, about 1.5 us of 3.6 a half-sweep at 400^2 (a release store to the counter
+// instead of the reduction: 4.5).
+__global__ void __launch_bounds__(32 * kLoopWarps, 1)
+jacobi2d_limb_loop(double* a, double* b, int64_t ny, int64_t nx, int halfsweeps, int strips,
+                   int chunk, int units, int near, uint32_t* __restrict__ done) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int unit = int(blockIdx.x) * int(blockDim.x >> 5) + warp;
+  const int64_t k0 = 1 + int64_t(unit % strips) * jlimb::kStrip, ib = 1 + int64_t(unit / strips) * chunk;
+  const int64_t ie = ib + chunk < ny - 1 ? ib + chunk : ny - 1;
+  const int cta = int(blockIdx.x) - near + lane;
+  const bool waits = warp == 0 && lane <= 2 * near && lane != near && cta >= 0 && cta < int(gridDim.x);
+  const jlimb::Limbs limbs{fxl::consts()};
+  for (int s = 0; s < halfsweeps; ++s) {
+    bool ok = true;
+    if (s > 0 && waits) {
+      uint64_t t0 = 0;
+      for (uint32_t n = 1;; ++n) {
+        uint32_t v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(done + cta) : "memory");
+        if (int32_t(v - uint32_t(s)) >= 0) break;
+        if ((n & 255u) == 0) {
+          const uint64_t now = tma::globaltimer();
+          if (t0 == 0) t0 = now;
+          if (now - t0 > kLoopLimitNs) {
+            atomicOr(&g_jacobi_tma_error, 2u);
+            ok = false;
+            break;
+          }
+        }
+      }
+    }
+    if (__syncthreads_or(!ok)) return;
+    const double* src = s & 1 ? b : a;
+    double* dst = s & 1 ? a : b;
+    if (unit < units && !jlimb::rows<jlimb::Limbs, true>(limbs, src, dst, nx, k0, ib, ie))
+      jlimb::rows_hardware<true>(src, dst, nx, k0, ib, ie);
+    __syncthreads();
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(done + blockIdx.x) : "memory");
+  }
 }
 
 // Warps per CTA and rows per warp, by q, the strips' rows per warp that the GPU holds at
@@ -154,6 +204,51 @@ int32_t run_limb(double* a, double* b, int64_t ny, int64_t nx, int32_t tsteps, c
       e = launch_chained(kern, grid, dim3{32u * unsigned(s.warps)}, 0, st, static_cast<const double*>(b), a, ny, nx, s.chunk);
   }
   return cuda_status(e, "jacobi2d_limb");
+}
+
+// NPBGB_ERR_STATE (nothing launched) where the chained launches are to be used.  The line
+// follows the units a CTA; in us, chained and in one launch, values in [0, 1) and then
+// standard normal ones: 2 (150^2, TSTEPS=50) 244, 274 and 306, 345; 10 (200 x 481, 20)
+// 147, 138 and 191, 166; 14 (350^2, 50) 377, 329 and 514, 413; 16 (300 x 481, 50) 342, 328
+// and 485, 437; 18 (400^2, 50) 391, 349 and 518, 466; 25 (480^2, 50) 412, 409 and 541, 548;
+// 32 (608 x 481, 30) 244, 274 and 325, 379.  Wider grids do not gain: 150 x 1000, 30, 197,
+// 229 and 269, 286; 200 x 700 212, 213 and 294, 277.
+int32_t run_limb_loop(double* a, double* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st) {
+  if (g_cfg_jacobi_bands != 1 || g_cfg_jacobi_chunk != 0 || tsteps < 16 || tsteps > (1 << 30)) return NPBGB_ERR_STATE;
+  constexpr int kChunk = 2;
+  const int64_t strips = cdiv(nx - 2, jlimb::kStrip), units = strips * cdiv(ny - 2, kChunk);
+  if (nx > 481 || units < 10 * int64_t(sm_count()) || units > kLoopWarps * int64_t(sm_count())) return NPBGB_ERR_STATE;
+  const int per_cta = int(cdiv(units, sm_count()));
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
+    return NPBGB_ERR_STATE;  // (the chained launches need no scratch memory)
+  const int nb = int(cdiv(units, per_cta)), near = int(cdiv(strips + 1, per_cta));
+  cudaMemPool_t pool;
+  void* scratch = nullptr;
+  cudaError_t e;
+  if ((e = scratch_pool(&pool)) != cudaSuccess ||
+      (e = cudaMallocFromPoolAsync(&scratch, size_t(nb) * sizeof(uint32_t), pool, st)) != cudaSuccess) {
+    cudaGetLastError();
+    return NPBGB_ERR_STATE;
+  }
+  e = cudaMemsetAsync(scratch, 0, size_t(nb) * sizeof(uint32_t), st);
+  if (e == cudaSuccess) {
+    auto* done = static_cast<uint32_t*>(scratch);
+    int hs = 2 * (tsteps - 1), strips_ = int(strips), chunk = kChunk, units_ = int(units), near_ = near;
+    void* args[] = {&a, &b, &ny, &nx, &hs, &strips_, &chunk, &units_, &near_, &done};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(nb));
+    cfg.blockDim = dim3(32u * unsigned(per_cta));
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = launch_together(cfg, reinterpret_cast<const void*>(jacobi2d_limb_loop), args);
+  }
+  cudaFreeAsync(scratch, st);
+  return cuda_status(e, "jacobi2d_limb_loop");
 }
 
 int pick_chunk(int64_t ny, int64_t col_blocks) {
@@ -205,8 +300,10 @@ int32_t run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st)
   if constexpr (FX) {
     // Limbs unless a setting of the other forms asks for one of those.
     if (g_cfg_jacobi_hw_warps < 0 && g_cfg_jacobi_tma != 2 && g_cfg_jacobi_fx_adds == 0 &&
-        g_cfg_jacobi_fx_mul == 1)
-      return run_limb(a, b, ny, nx, tsteps, st);
+        g_cfg_jacobi_fx_mul == 1) {
+      const int32_t r = run_limb_loop(a, b, ny, nx, tsteps, st);
+      return r != NPBGB_ERR_STATE ? r : run_limb(a, b, ny, nx, tsteps, st);
+    }
   }
   const int64_t gx = cdiv(nx - 2, 32 * kWarps);
   const int chunk = pick_chunk(ny, gx);

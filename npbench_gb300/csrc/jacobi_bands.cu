@@ -37,8 +37,8 @@
 // Bound by the instructions of a point and by the hand-off's latency: a half-sweep of
 // binary32 1403 x 1177 takes 2.2 us where the points alone take about 1.5.  Measured,
 // chained launches to bands, TSTEPS=100: binary32 1000^2 0.72 to 0.40 ms, 1403 x 1177
-// 1.02 to 0.48, 2048^2 (TSTEPS=50) 0.785 to 0.39; binary64 300^2 (50) 0.36 to 0.25,
-// 1000^2 1.68 to 1.5.  With every edge through L2 the 1403 x 1177 grid took 0.85 ms,
+// 1.02 to 0.48, 2048^2 (TSTEPS=50) 0.785 to 0.39; binary64 on values in [0, 1) 300^2 (50)
+// 0.30 to 0.25.  With every edge through L2 the 1403 x 1177 grid took 0.85 ms,
 // with the computing threads polling instead of extra warps 0.71.
 //
 // Places of edge values alternate between two slots.  A thread sends sweep s+1 of a
@@ -882,10 +882,10 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
 // binary64, 4096 of binary32), on a stream that is being captured (the chained kernels
 // need no scratch memory), and, unless asked for every grid that fits
 // (NPBGB_CFG_JACOBI_BANDS = 2), where the chained kernels measured faster:
-//   * binary64 other than up to 481 columns and 2 pairs a thread.  There bands take
-//     0.25 against 0.36 ms (300^2, TSTEPS=50); larger grids win less on values in
-//     range (700^2, TSTEPS=100: 0.95 against 1.23) than they lose where every value
-//     is out of the limbs' range (TSTEPS=50: 1.50 against 0.95);
+//   * binary64: on values in [0, 1) bands win (300^2, TSTEPS=50: 0.25 against 0.30 ms),
+//     but every pair with a value out of the limbs' range is mended out of line, and
+//     fields come to hold such values (NPBench's own initial field 0.63 against 0.35, a
+//     hot wall in a cold box 0.51 against 0.33, standard normal values 0.64 against 0.39);
 //   * binary32 of more than 2049 columns (8 a thread) with 2 pairs a thread: 300 x
 //     2990, TSTEPS=50 0.461 against 0.447 ms (700 x 2900 0.481 against 0.586);
 //   * short runs, as launch, load and way back cost about 25 us and more for wide
@@ -896,7 +896,7 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   if (g_cfg_jacobi_bands == 0) return NPBGB_ERR_STATE;
   const bool any = g_cfg_jacobi_bands == 2;
   if (tsteps <= 1 || ny < 4 || nx < 3 || ny > (1 << 20) || nx > 4096) return NPBGB_ERR_STATE;
-  if (sizeof(T) == 8 && !g_cfg_f64_emulation) return NPBGB_ERR_STATE;
+  if (sizeof(T) == 8 && !(any && g_cfg_f64_emulation)) return NPBGB_ERR_STATE;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
     return NPBGB_ERR_STATE;
@@ -908,7 +908,7 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   // As few columns a thread as the width allows.
   int which = 0;
   while (which < 3 && nx - 1 > int64_t(instances<T>()[which].cpt) * instances<T>()[which].compute) ++which;
-  if (which == 3 || (sizeof(T) == 8 && !any && which > 0)) return NPBGB_ERR_STATE;
+  if (which == 3) return NPBGB_ERR_STATE;
   const Instance<T>& in = instances<T>()[which];
   const int compute = int(cdiv(cdiv(nx - 1, in.cpt), 32) * 32), columns = in.cpt * compute;
   // As few pairs a thread as any cluster size gives, but two (one leaves more bands
@@ -925,7 +925,7 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   const size_t smem = in_cluster ? in.bytes(H, compute) : 0;
   if (in_cluster == 0 || smem > room) return NPBGB_ERR_STATE;
   const bool wide = sizeof(T) == 4 && which == 2;
-  if (!any && (tsteps < (wide ? 16 : 8) || (sizeof(T) == 8 && H > 2) || (wide && H < 3))) return NPBGB_ERR_STATE;
+  if (!any && (tsteps < (wide ? 16 : 8) || (wide && H < 3))) return NPBGB_ERR_STATE;
   const int nb = int(cdiv(interior, 2 * H)), clusters = int(cdiv(nb, in_cluster));
   const size_t mail_bytes = size_t(4) * clusters * size_t(columns) * sizeof(typename Kind<T>::Mail);
   const size_t bytes = mail_bytes + 256;  // and a counter

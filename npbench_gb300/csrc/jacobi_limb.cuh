@@ -31,8 +31,15 @@ using fxl::P2;
 __device__ __forceinline__ double hardware(double c, double w, double e, double s, double n) {
   return mul_rn(0.2, add_rn(add_rn(add_rn(add_rn(c, w), e), s), n));
 }
+// CG here and below: loads go through the L2, for arrays that other CTAs of the same launch
+// write.
+template <bool CG>
+__device__ __forceinline__ double load(const double* p) {
+  if constexpr (CG) return __ldcg(p); else return *p;
+}
+template <bool CG>
 static __device__ __noinline__ double hardware_point(const double* p, int64_t nx) {
-  return hardware(p[0], p[-1], p[1], p[nx], p[-nx]);
+  return hardware(load<CG>(p), load<CG>(p - 1), load<CG>(p + 1), load<CG>(p + nx), load<CG>(p - nx));
 }
 
 // The two arithmetics of a pair.
@@ -97,7 +104,7 @@ __device__ __forceinline__ uint32_t finite_word(double x) {
 
 // Output rows [r0, r1) at columns k0 .. k0 + 29 (warp-collective).  False, and nothing
 // written, if M is Limbs and the strip wants Hardware.
-template <class M>
+template <class M, bool CG = false>
 __device__ __forceinline__ bool rows(M m, const double* __restrict__ src, double* __restrict__ dst, int64_t nx,
                                      int64_t k0, int64_t r0, int64_t r1) {
   using Pair = typename M::Pair;
@@ -115,21 +122,21 @@ __device__ __forceinline__ bool rows(M m, const double* __restrict__ src, double
   int q = 0;
   double ra, rb;
   const bool odd = (count & 1) != 0;
-  auto load = [&]() {
-    ra = in ? p[0] : 0.0;
-    rb = in ? p[odd && q > half ? apart - nx : apart] : 0.0;
+  auto next = [&]() {
+    ra = in ? load<CG>(p) : 0.0;
+    rb = in ? load<CG>(p + (odd && q > half ? apart - nx : apart)) : 0.0;
     p += nx;
     ++q;
   };
-  load();
+  next();
   const double za = ra, zb = rb;
-  load();
+  next();
   if constexpr (kLimbs) {
     const uint32_t wa = finite_word(ra), wb = finite_word(rb);
     m.K.scale = fxl::frame_of(__reduce_max_sync(0xffffffffu, wa > wb ? wa : wb));
   }
   Pair x0 = m.from(za, zb), x1 = m.from(ra, rb), x2;
-  load();
+  next();
   if constexpr (kLimbs) {
     const bool lost = fxl::refused_value(x0) || fxl::refused_value(x1);
     if (__popc(__ballot_sync(0xffffffffu, lost)) > 8) return false;
@@ -137,7 +144,7 @@ __device__ __forceinline__ bool rows(M m, const double* __restrict__ src, double
   int i = 0;
   auto step = [&](const Pair& xp, const Pair& xc, Pair& xn) -> bool {
     xn = m.from(ra, rb);
-    if (i + 1 < half) load();
+    if (i + 1 < half) next();
     double va, vb;
     m.point(xc, xn, xp, va, vb);
     const bool second = i + half < count;
@@ -145,8 +152,8 @@ __device__ __forceinline__ bool rows(M m, const double* __restrict__ src, double
       if (!(m.sure_a && m.sure_b)) {
         const double* at = src + (o - dst);
         // the limbs of a zero sum's product are zero
-        if (!m.sure_a) va = out && fxl::first(m.t) != 0u ? hardware_point(at, nx) : 0.0;
-        if (!m.sure_b) vb = out && second && fxl::second(m.t) != 0u ? hardware_point(at + apart, nx) : 0.0;
+        if (!m.sure_a) va = out && fxl::first(m.t) != 0u ? hardware_point<CG>(at, nx) : 0.0;
+        if (!m.sure_b) vb = out && second && fxl::second(m.t) != 0u ? hardware_point<CG>(at + apart, nx) : 0.0;
       }
     }
     if (out) {
@@ -161,9 +168,10 @@ __device__ __forceinline__ bool rows(M m, const double* __restrict__ src, double
   return true;
 }
 
+template <bool CG = false>
 static __device__ __noinline__ void rows_hardware(const double* __restrict__ src, double* __restrict__ dst, int64_t nx,
-                                           int64_t k0, int64_t r0, int64_t r1) {
-  rows(Hardware{}, src, dst, nx, k0, r0, r1);
+                                                  int64_t k0, int64_t r0, int64_t r1) {
+  rows<Hardware, CG>(Hardware{}, src, dst, nx, k0, r0, r1);
 }
 
 }  // namespace jlimb
