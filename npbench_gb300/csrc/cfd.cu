@@ -916,6 +916,9 @@ struct MailPlan {
   int threads = 0, per_thread = 0;
   size_t smem = 0;
 };
+// Elements are stored and loaded whole; a workspace that is only aligned for doubles takes
+// cfd_bands.
+bool mail_aligned(const void* workspace) { return reinterpret_cast<uintptr_t>(workspace) % sizeof(ulonglong2) == 0; }
 constexpr size_t kMailSmem = 190 * 1024;  // next to the deciding CTA's static 33 KB
 
 MailPlan mail_plan(int64_t ny, int64_t nx, bool channel) {
@@ -1032,7 +1035,7 @@ extern "C" int32_t npbgb_cavity_flow(void* u, void* v, void* p, int64_t ny, int6
   int32_t status = NPBGB_OK;
   cudaError_t e = cudaSuccess;
   const MailPlan m = mail_plan(ny, nx, false);
-  if (m.fits && (workspace == nullptr || workspace_bytes >= m.p_bytes + m.uv_bytes)) {
+  if (m.fits && mail_aligned(w) && (workspace == nullptr || workspace_bytes >= m.p_bytes + m.uv_bytes)) {
     a.p_mail = reinterpret_cast<ulonglong2*>(w);
     a.uv_mail = reinterpret_cast<ulonglong2*>(w + m.p_bytes);
     a.nbands = int32_t(m.nb);
@@ -1232,7 +1235,7 @@ extern "C" int32_t npbgb_channel_flow(void* u, void* v, void* p, int64_t ny, int
       channel_small<<<1, kCThreads, 0, st>>>(a);
       e = counted(cudaGetLastError());
     } else if (const MailPlan m = mail_plan(ny, nx, true);
-               m.fits && (workspace == nullptr || workspace_bytes >= l.total)) {
+               m.fits && mail_aligned(w) && (workspace == nullptr || workspace_bytes >= l.total)) {
       a.p_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail);
       a.uv_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail + m.p_bytes);
       a.nbands = int32_t(m.nb);
