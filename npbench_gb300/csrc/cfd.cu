@@ -492,8 +492,11 @@ __device__ __forceinline__ bool collect(const ulonglong2* const (&at)[N], bool (
   }
 }
 
-// Channel flow's verdicts.  ctl counts the steps that may change u and v.
+// Channel flow's verdicts.  ctl counts the steps that may change u and v.  One of its waits
+// covers a whole step, so its limit grows with the step's pressure iterations (a sweep
+// takes 1.2 us, at most 20 with the longest bands).
 __device__ void channel_verdict(const CfdArgs& a) {
+  const uint64_t limit_ns = kCfdLimitNs + uint64_t(a.nit) * 100000ull;
   double s_prev = numpy_sum_cta(a, a.u[0]);
   if (threadIdx.x == 0) st_release(a.ctl, 1u);
   for (uint32_t n = 1;; ++n) {
@@ -501,7 +504,7 @@ __device__ void channel_verdict(const CfdArgs& a) {
     const uint64_t t0 = globaltimer();
     for (int bb = threadIdx.x; bb < a.nbands && r; bb += int(blockDim.x))
       while (ld_acquire(a.done + bb) < n)
-        if (globaltimer() - t0 > kCfdLimitNs) {
+        if (globaltimer() - t0 > limit_ns) {
           atomicOr(&g_cfd_error, 1u);
           r = 0;
           break;
