@@ -221,8 +221,10 @@ NPBGB_API int32_t npbgb_selftest_wait_timeout(int64_t limit_ns, void* stream);
 
 /* How the calling thread's next cooperative launch is made: 0 as always,
  * NPBGB_LAUNCH_UNCLUSTERED without its cluster dimension, as Nsight Compute
- * makes it.  The results must not differ.  No counterpart in the reference. */
+ * makes it, NPBGB_LAUNCH_REFUSED not at all, as where its CTAs do not all find
+ * an SM.  The results must not differ.  No counterpart in the reference. */
 #define NPBGB_LAUNCH_UNCLUSTERED 1
+#define NPBGB_LAUNCH_REFUSED 2
 NPBGB_API int32_t npbgb_selftest_launch(int32_t how);
 
 /* Converts n elements: NPBGB_F32 -> NPBGB_F64 (exact) or NPBGB_F64 -> NPBGB_F32

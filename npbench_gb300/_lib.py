@@ -46,6 +46,7 @@ NPBGB_CFG_JACOBI_FX_ADDS = 25
 NPBGB_CFG_JACOBI_TMA = 26
 NPBGB_CFG_BATCH_TMA = 27
 NPBGB_LAUNCH_UNCLUSTERED = 1
+NPBGB_LAUNCH_REFUSED = 2
 NPBGB_BATCH_PERSISTENT = 1
 NPBGB_BATCH_STEPPED = 2
 NPBGB_BATCH_QUEUE = 3

@@ -70,6 +70,7 @@ static thread_local int32_t g_next_launch = 0;
 cudaError_t launch_together(const cudaLaunchConfig_t& cfg, const void* kernel, void** args) {
   const int32_t how = g_next_launch;
   g_next_launch = 0;
+  if (how == NPBGB_LAUNCH_REFUSED) return cudaErrorCooperativeLaunchTooLarge;
   cudaLaunchAttribute attr[4];
   cudaLaunchConfig_t c = cfg;
   if (how == NPBGB_LAUNCH_UNCLUSTERED) {
@@ -78,7 +79,9 @@ cudaError_t launch_together(const cudaLaunchConfig_t& cfg, const void* kernel, v
     for (unsigned n = 0; n < cfg.numAttrs; ++n)
       if (cfg.attrs[n].id != cudaLaunchAttributeClusterDimension) attr[c.numAttrs++] = cfg.attrs[n];
   }
-  return counted(cudaLaunchKernelExC(&c, kernel, args));
+  const cudaError_t e = counted(cudaLaunchKernelExC(&c, kernel, args));
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 namespace tma {
@@ -321,7 +324,8 @@ int32_t npbgb_selftest_wait_timeout(int64_t limit_ns, void* stream) {
 
 int32_t npbgb_selftest_launch(int32_t how) {
   using namespace npbgb;
-  if (how != 0 && how != NPBGB_LAUNCH_UNCLUSTERED) return set_error(NPBGB_ERR_ARG, "unknown kind of launch %d", how);
+  if (how != 0 && how != NPBGB_LAUNCH_UNCLUSTERED && how != NPBGB_LAUNCH_REFUSED)
+    return set_error(NPBGB_ERR_ARG, "unknown kind of launch %d", how);
   g_next_launch = how;
   return NPBGB_OK;
 }

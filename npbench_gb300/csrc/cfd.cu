@@ -953,7 +953,7 @@ cudaError_t launch_cooperative(const void* kernel, unsigned ctas, unsigned threa
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   void* args[] = {&a};
-  return npbgb::counted(cudaLaunchKernelExC(&cfg, kernel, args));
+  return npbgb::launch_together(cfg, kernel, args);
 }
 
 // The kernel for a plan, ready to launch cooperatively; nullptr with `e` set on failure.
@@ -1038,16 +1038,19 @@ extern "C" int32_t npbgb_cavity_flow(void* u, void* v, void* p, int64_t ny, int6
   int32_t status = NPBGB_OK;
   cudaError_t e = cudaSuccess;
   const MailPlan m = mail_plan(ny, nx, false);
+  bool launched = false;  // where the mailbox form's launch is refused, the band form's is tried
   if (m.fits && mail_aligned(w) && (workspace == nullptr || workspace_bytes >= m.p_bytes + m.uv_bytes)) {
-    a.p_mail = reinterpret_cast<ulonglong2*>(w);
-    a.uv_mail = reinterpret_cast<ulonglong2*>(w + m.p_bytes);
-    a.nbands = int32_t(m.nb);
-    a.rows = int32_t(m.rows);
+    CfdArgs c = a;
+    c.p_mail = reinterpret_cast<ulonglong2*>(w);
+    c.uv_mail = reinterpret_cast<ulonglong2*>(w + m.p_bytes);
+    c.nbands = int32_t(m.nb);
+    c.rows = int32_t(m.rows);
     e = cudaMemsetAsync(w, 0, size_t(m.p_bytes + m.uv_bytes), st);
     const void* kern = e == cudaSuccess ? mail_kernel<false>(m, e) : nullptr;
-    if (kern) e = launch_cooperative(kern, unsigned(m.nb), unsigned(m.threads), m.smem, st, a);
-  } else {
-    e = cudaMemsetAsync(a.done, 0, size_t(nb) * sizeof(uint32_t), st);
+    launched = kern && launch_cooperative(kern, unsigned(m.nb), unsigned(m.threads), m.smem, st, c) == cudaSuccess;
+  }
+  if (!launched) {
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.done, 0, size_t(nb) * sizeof(uint32_t), st);
     if (e == cudaSuccess)
       e = launch_cooperative(reinterpret_cast<const void*>(cfd_bands<false>), unsigned(nb),
                              unsigned(kCThreads), 0, st, a);
@@ -1237,18 +1240,22 @@ extern "C" int32_t npbgb_channel_flow(void* u, void* v, void* p, int64_t ny, int
     if (ny < 3) {
       channel_small<<<1, kCThreads, 0, st>>>(a);
       e = counted(cudaGetLastError());
-    } else if (const MailPlan m = mail_plan(ny, nx, true);
-               m.fits && mail_aligned(w) && (workspace == nullptr || workspace_bytes >= l.total)) {
-      a.p_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail);
-      a.uv_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail + m.p_bytes);
-      a.nbands = int32_t(m.nb);
-      a.rows = int32_t(m.rows);
-      e = cudaMemsetAsync(w + l.off_mail, 0, size_t(m.p_bytes + m.uv_bytes), st);
-      const void* kern = e == cudaSuccess ? mail_kernel<true>(m, e) : nullptr;
-      if (kern) e = launch_cooperative(kern, unsigned(m.nb + 1), unsigned(m.threads), m.smem, st, a);
     } else {
-      e = launch_cooperative(reinterpret_cast<const void*>(cfd_bands<true>), unsigned(l.nb),
-                             unsigned(kCThreads), 0, st, a);
+      const MailPlan m = mail_plan(ny, nx, true);
+      bool launched = false;  // (as in cavity flow)
+      if (m.fits && mail_aligned(w) && (workspace == nullptr || workspace_bytes >= l.total)) {
+        CfdArgs c = a;
+        c.p_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail);
+        c.uv_mail = reinterpret_cast<ulonglong2*>(w + l.off_mail + m.p_bytes);
+        c.nbands = int32_t(m.nb);
+        c.rows = int32_t(m.rows);
+        e = cudaMemsetAsync(w + l.off_mail, 0, size_t(m.p_bytes + m.uv_bytes), st);
+        const void* kern = e == cudaSuccess ? mail_kernel<true>(m, e) : nullptr;
+        launched = kern && launch_cooperative(kern, unsigned(m.nb + 1), unsigned(m.threads), m.smem, st, c) == cudaSuccess;
+      }
+      if (!launched && e == cudaSuccess)
+        e = launch_cooperative(reinterpret_cast<const void*>(cfd_bands<true>), unsigned(l.nb),
+                               unsigned(kCThreads), 0, st, a);
     }
   }
   if (e == cudaSuccess && steps != nullptr) {

@@ -158,7 +158,7 @@ jacobi1d_resident(float* __restrict__ A, float* __restrict__ B, int64_t n, int h
 }  // namespace
 
 // NPBGB_ERR_STATE (nothing launched; the caller then uses the chained launches) when
-// the CTAs that fit one per SM cannot hold the array, or on a stream that is being
+// the CTAs that fit one per SM cannot hold the array, when the launch is refused, or on a stream that is being
 // captured (the chained launches need no scratch memory).
 int32_t jacobi1d_resident_run(float* a, float* b, int64_t n, int32_t tsteps, cudaStream_t st) {
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -194,10 +194,10 @@ int32_t jacobi1d_resident_run(float* a, float* b, int64_t n, int32_t tsteps, cud
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    e = counted(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(jacobi1d_resident), args));
+    e = launch_together(cfg, reinterpret_cast<const void*>(jacobi1d_resident), args);
   }
   cudaFreeAsync(scratch, st);
-  return cuda_status(e, "jacobi1d_resident");
+  return e == cudaSuccess ? NPBGB_OK : NPBGB_ERR_STATE;  // not launched
 }
 
 uint32_t take_jacobi1d_device_error() {

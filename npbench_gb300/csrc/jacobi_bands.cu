@@ -960,7 +960,7 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
     e = launch_together(cfg, reinterpret_cast<const void*>(in.kern), args);
   }
   cudaFreeAsync(scratch, st);
-  return cuda_status(e, "jacobi2d_bands");
+  return e == cudaSuccess ? NPBGB_OK : NPBGB_ERR_STATE;  // not launched
 }
 
 template int32_t jacobi2d_bands_run<double>(double*, double*, int64_t, int64_t, int32_t, cudaStream_t);

@@ -106,7 +106,9 @@ inline cudaError_t counted(cudaError_t e) {
   return e;
 }
 
-// A counted cooperative launch (npbgb_selftest_launch can change the next one).
+// A counted cooperative launch (npbgb_selftest_launch can change the next one).  An error is
+// returned and not left behind: where the CTAs cannot all be resident, in a process that
+// has fewer SMs than the device, say, callers have a form that needs fewer or none.
 cudaError_t launch_together(const cudaLaunchConfig_t& cfg, const void* kernel, void** args);
 
 extern int64_t g_cfg_hdiff_emu;  // NPBGB_CFG_HDIFF_EMU
