@@ -169,7 +169,7 @@ int32_t jacobi1d_resident_run(float* a, float* b, int64_t n, int32_t tsteps, cud
   // 0.87 at N=32000).
   const int64_t w = std::max<int64_t>(cdiv(n - 2, sm_count()), 148);
   const int H = int(std::min<int64_t>((kSpan - w) / 2, w)) & ~3;
-  if (H < 32) return NPBGB_ERR_STATE;
+  if (H < 32 || tsteps > (1 << 30)) return NPBGB_ERR_STATE;  // (half-sweeps are counted in 32 bits)
   const int nb = int(cdiv(n - 2, w));
   const size_t bytes = size_t(4) * nb * size_t(H) * sizeof(Mail);
   cudaMemPool_t pool;

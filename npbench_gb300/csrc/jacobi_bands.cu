@@ -895,7 +895,7 @@ template <typename T>
 int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st) {
   if (g_cfg_jacobi_bands == 0) return NPBGB_ERR_STATE;
   const bool any = g_cfg_jacobi_bands == 2;
-  if (tsteps <= 1 || ny < 4 || nx < 3 || ny > (1 << 20) || nx > 4096) return NPBGB_ERR_STATE;
+  if (tsteps <= 1 || tsteps > (1 << 30) || ny < 4 || nx < 3 || ny > (1 << 20) || nx > 4096) return NPBGB_ERR_STATE;
   if (sizeof(T) == 8 && !(any && g_cfg_f64_emulation)) return NPBGB_ERR_STATE;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
