@@ -1039,7 +1039,10 @@ extern "C" int32_t npbgb_cavity_flow(void* u, void* v, void* p, int64_t ny, int6
   cudaError_t e = cudaSuccess;
   const MailPlan m = mail_plan(ny, nx, false);
   bool launched = false;  // where the mailbox form's launch is refused, the band form's is tried
-  if (m.fits && mail_aligned(w) && (workspace == nullptr || workspace_bytes >= m.p_bytes + m.uv_bytes)) {
+  // Next to a tile queue's worker, mailbox CTAs of more than 22 KB found no room on an SM
+  // (201 x 201 did, 330 x 200 and 100 x 500 did not); the band form's do.
+  const bool room = !queue_exists() || (m.per_thread == 1 && m.smem <= 22 * 1024 + 512);
+  if (m.fits && room && mail_aligned(w) && (workspace == nullptr || workspace_bytes >= m.p_bytes + m.uv_bytes)) {
     CfdArgs c = a;
     c.p_mail = reinterpret_cast<ulonglong2*>(w);
     c.uv_mail = reinterpret_cast<ulonglong2*>(w + m.p_bytes);

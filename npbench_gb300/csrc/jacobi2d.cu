@@ -214,7 +214,8 @@ int32_t run_limb(double* a, double* b, int64_t ny, int64_t nx, int32_t tsteps, c
 // 32 (608 x 481, 30) 244, 274 and 325, 379.  Wider grids do not gain: 150 x 1000, 30, 197,
 // 229 and 269, 286; 200 x 700 212, 213 and 294, 277.
 int32_t run_limb_loop(double* a, double* b, int64_t ny, int64_t nx, int32_t tsteps, cudaStream_t st) {
-  if (g_cfg_jacobi_bands != 1 || g_cfg_jacobi_chunk != 0 || tsteps < 16 || tsteps > (1 << 30)) return NPBGB_ERR_STATE;
+  if (g_cfg_jacobi_bands != 1 || g_cfg_jacobi_chunk != 0 || tsteps < 16 || tsteps > (1 << 30) || queue_exists())
+    return NPBGB_ERR_STATE;
   constexpr int kChunk = 2;
   const int64_t strips = cdiv(nx - 2, jlimb::kStrip), units = strips * cdiv(ny - 2, kChunk);
   if (nx > 481 || units < 10 * int64_t(sm_count()) || units > kLoopWarps * int64_t(sm_count())) return NPBGB_ERR_STATE;

@@ -888,6 +888,7 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
 //     hot wall in a cold box 0.51 against 0.33, standard normal values 0.64 against 0.39);
 //   * binary32 of more than 2049 columns (8 a thread) with 2 pairs a thread: 300 x
 //     2990, TSTEPS=50 0.461 against 0.447 ms (700 x 2900 0.481 against 0.586);
+//   * next to a tile queue, whose worker would keep the bands' CTAs waiting;
 //   * short runs, as launch, load and way back cost about 25 us and more for wide
 //     grids (binary32, TSTEPS=6 and 11: 1000^2 52 and 69 us against 55 and 91; 2500^2
 //     164 and 227 against 123 and 229, with 21 358 against 436).
@@ -897,6 +898,7 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   const bool any = g_cfg_jacobi_bands == 2;
   if (tsteps <= 1 || tsteps > (1 << 30) || ny < 4 || nx < 3 || ny > (1 << 20) || nx > 4096) return NPBGB_ERR_STATE;
   if (sizeof(T) == 8 && !(any && g_cfg_f64_emulation)) return NPBGB_ERR_STATE;
+  if (!any && queue_exists()) return NPBGB_ERR_STATE;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
     return NPBGB_ERR_STATE;

@@ -111,6 +111,12 @@ inline cudaError_t counted(cudaError_t e) {
 // has fewer SMs than the device, say, callers have a form that needs fewer or none.
 cudaError_t launch_together(const cudaLaunchConfig_t& cfg, const void* kernel, void** args);
 
+// Whether a tile queue exists on the current device (queue.cu).  Its worker kernel stays on
+// the SMs for as long as grids arrive, and a launch whose CTAs need more registers or
+// shared memory than it leaves waits for all that time (with one worker CTA an SM: 34
+// thousand registers, and the shared memory that the SM was set up for).
+bool queue_exists();
+
 extern int64_t g_cfg_hdiff_emu;  // NPBGB_CFG_HDIFF_EMU
 
 // allow_pdl = false launches in plain stream order whatever NPBGB_CFG_PDL says

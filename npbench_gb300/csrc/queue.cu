@@ -53,6 +53,7 @@
 // polybench/heat_3d/heat_3d_numpy.py:6-20), binary64 fixed-point paths
 // included.
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <new>
@@ -596,6 +597,18 @@ struct npbgb_queue {
   std::mutex mu;
 };
 
+namespace npbgb {
+static std::atomic<int> g_queues[64];  // per device
+
+bool queue_exists() {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && g_queues[dev].load() > 0;
+}
+static void count_queue(int dev, int n) {
+  if (dev >= 0 && dev < 64) g_queues[dev].fetch_add(n);
+}
+}  // namespace npbgb
+
 namespace {
 
 void free_queue(npbgb_queue* q) {
@@ -699,6 +712,7 @@ int32_t npbgb_queue_create(int32_t max_slots, int32_t tile_rows, int32_t tile_pl
   q->gen.assign(size_t(max_slots), 0u);
   q->busy.assign(size_t(max_slots), 0);
   for (int32_t s = max_slots - 1; s >= 0; --s) q->free_slots.push_back(s);
+  count_queue(q->device, 1);
   *out = q;
   return NPBGB_OK;
 }
@@ -820,6 +834,7 @@ int32_t npbgb_queue_destroy(npbgb_queue* q) {
     store_release(q->h_ctl + 1, 1u);
     if (q->launched) cudaEventSynchronize(q->done_ev);  // ends: closed, and bounded waits
   }
+  count_queue(q->device, -1);
   free_queue(q);
   return NPBGB_OK;
 }
