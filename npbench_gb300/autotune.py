@@ -7,8 +7,8 @@
     python -m npbench_gb300.autotune --ship FILE      # all of the above into FILE
 
 The kernels take knobs that change speed, never results (``NPBGB_CFG_*``): for
-binary64 Jacobi-2D the warps per CTA on the hardware binary64 path, the
-rows per CTA and whether the whole loop runs in one launch with bands of rows
+binary64 Jacobi-2D the warps per CTA on the hardware binary64 path (of the
+fixed-point form; none selects the limb form), the rows per CTA and whether the whole loop runs in one launch with bands of rows
 in shared memory; for Heat-3D the tile rows per warp, the rows on hardware
 binary64, the planes per CTA and, in binary32, the half-sweeps per launch
 (temporal depth, 1 or 2).  Batches have their tile rows and hardware warps;
@@ -24,7 +24,7 @@ the server has one class per stream description.
 candidate with CUDA events, check that each leaves exactly the bits of the
 default (the knobs must not change results; a mismatch raises) and store the
 fastest.  Lookups read the user cache (NPBGB_TUNE_CACHE, else
-~/.cache/npbench_gb300/tune.json) and then ``tuned.json`` shipped in this
+~/.cache/npbench_gb300/tune.json), but for entries of other versions of the library, and then ``tuned.json`` shipped in this
 package, measured on GB300 by ``--ship``.  Tuned settings are applied by
 default; NPBGB_AUTOTUNE=0 in the environment, or ``disable()``, turns that off.
 """
@@ -68,8 +68,10 @@ def _space(bench, dtype):
     f64 = np.dtype(dtype) == np.float64
     out = []
     if bench == "jacobi_2d":
-        for hw in ((0, 2, 3, 4, 5, 6, 8) if f64 else (-1,)):
-            for ch in (0, 3, 4, 6, 8, 16, 32):
+        # binary64: -1 is the limb form, whose rows go in pairs; the others the fixed-point
+        # form (all eight warps in hardware were never the fastest)
+        for hw in ((-1, 0, 2, 3, 4, 5, 6) if f64 else (-1,)):
+            for ch in ((0, 2, 4, 6, 10, 16, 24) if f64 and hw < 0 else (0, 3, 4, 6, 8, 16, 32)):
                 cfg = {"JACOBI_HW_WARPS": hw, "JACOBI_CHUNK": ch}
                 if f64:
                     cfg["JACOBI_BANDS"] = 0  # chained launches
@@ -82,9 +84,13 @@ def _space(bench, dtype):
                     out.append({"JACOBI_HW_WARPS": hw, "JACOBI_CHUNK": ch, "JACOBI_BANDS": 0,
                                 "JACOBI_TMA": 2})
     elif bench == "heat_3d":
-        if f64:  # the limb form, which has one setting; the rows select the integer form
-            for ch in (0, 1, 2, 3, 4, 6, 8, 10, 12, 16):
-                out.append({"HEAT_ROWS": 0, "HEAT_HW_ROWS": -1, "HEAT_CHUNK": ch})
+        # the limb form and, in binary32, the one by rows, which have one setting; rows
+        # (below) select the integer and TMA forms
+        for ch in (0, 1, 2, 3, 4, 6, 8, 10, 12, 16) if f64 else (0, 1, 2, 3, 4, 5, 6, 8):
+            cfg = {"HEAT_ROWS": 0, "HEAT_HW_ROWS": -1, "HEAT_CHUNK": ch}
+            if not f64:
+                cfg["HEAT_TB"] = 1
+            out.append(cfg)
         for rows in (1, 2, 4):
             tj = 8 * rows
             for hw in (sorted({0, tj // 8, tj // 4, 5 * tj // 16, 3 * tj // 8, 7 * tj // 16})
@@ -141,9 +147,14 @@ def load_cache(refresh=False):
 
 
 def lookup(k):
-    """The entry for key k: the user cache first, then the shipped table."""
-    cache = load_cache()
-    return cache.get(k) or _state["shipped"].get(k)
+    """The entry for key k: the user cache first, then the shipped table.
+
+    An entry that another version of the library was timed with is passed over: its setting
+    may name a form that has been replaced since."""
+    entry = load_cache().get(k)
+    if entry and entry.get("library", _lib.version()) != _lib.version():
+        entry = None
+    return entry or _state["shipped"].get(k)
 
 
 def _store(k, entry, path=None):
@@ -220,8 +231,10 @@ def tune(bench, shape, dtype, tsteps=None, repeats=3, space=None, store=True, pa
     """Times every candidate setting for (bench, shape, dtype); returns the cache entry
     (stored under the shape's class).
 
-    Each candidate must leave exactly the bits the default setting leaves (else
-    RuntimeError).  tsteps defaults to 21 (40 half-sweeps).
+    A candidate's time is the mean over two fields, values in [0, 1) and NPBench's own
+    initial field (values beyond 1): the binary64 forms' speed depends on the values.  Each
+    candidate must leave exactly the bits the default setting leaves (else RuntimeError).
+    tsteps defaults to 21 (40 half-sweeps).
     """
     import torch
 
@@ -232,46 +245,52 @@ def tune(bench, shape, dtype, tsteps=None, repeats=3, space=None, store=True, pa
     shape = tuple(int(s) for s in shape)
     dtype = np.dtype(_dtype_name(dtype))
     kern = {"jacobi_2d": stencils.jacobi_2d_kernel, "heat_3d": stencils.heat_3d_kernel}[bench]
+    at = np.indices(shape, sparse=True)
     if bench == "jacobi_2d":
-        A0, B0 = workloads.uniform_pair(shape, dtype.type, seed=1)
+        pairs = [workloads.uniform_pair(shape, dtype.type, seed=1),
+                 (at[0] * (at[1] + 2) / shape[0], at[0] * (at[1] + 3) / shape[0])]
     else:
-        A0, B0 = workloads.uniform_heat(shape, dtype.type, seed=1)
+        ramp = (at[0] + at[1] + (shape[0] - at[2])) * 10 / shape[0]
+        pairs = [workloads.uniform_heat(shape, dtype.type, seed=1), (ramp, ramp)]
     T = int(tsteps) if tsteps else 21
-    pA, pB = torch.from_numpy(A0).to(dev), torch.from_numpy(B0).to(dev)
-    A, B = torch.empty_like(pA), torch.empty_like(pB)
+    fields = [tuple(torch.from_numpy(x.astype(dtype)).to(dev) for x in pair) for pair in pairs]
+    A, B = torch.empty_like(fields[0][0]), torch.empty_like(fields[0][1])
     was_enabled = _state["enabled"]
     _state["enabled"] = False  # the kernels must see exactly the settings below
 
-    def run():
-        A.copy_(pA)
-        B.copy_(pB)
+    def run(field):
+        A.copy_(field[0])
+        B.copy_(field[1])
         kern(T, A, B)
 
     def timed():
-        run()
-        torch.cuda.synchronize(dev)
-
-        def once():
-            kern(T, A, B)
-        ms = []
-        for _ in range(repeats):
-            A.copy_(pA)
-            B.copy_(pB)
-            ms.append(_events_ms(once, dev, 1))
-        return float(np.median(ms))
+        total = 0.0
+        for field in fields:
+            run(field)
+            torch.cuda.synchronize(dev)
+            ms = []
+            for _ in range(repeats):
+                A.copy_(field[0])
+                B.copy_(field[1])
+                ms.append(_events_ms(lambda: kern(T, A, B), dev, 1))
+            total += float(np.median(ms))
+        return total / len(fields)
 
     try:
         base_cfg = _defaults(bench, dtype)
-        run()
-        ref = (A.clone(), B.clone())
+        refs = []
+        for field in fields:
+            run(field)
+            refs.append((A.clone(), B.clone()))
         base_ms = timed()
         results = []
         for cfg in (space or _space(bench, dtype)):
             with _settings(cfg):
-                run()
-                if not (torch.equal(A.view(torch.int8), ref[0].view(torch.int8)) and
-                        torch.equal(B.view(torch.int8), ref[1].view(torch.int8))):
-                    raise RuntimeError(f"setting {cfg} changed the results of {bench}")
+                for field, ref in zip(fields, refs):
+                    run(field)
+                    if not (torch.equal(A.view(torch.int8), ref[0].view(torch.int8)) and
+                            torch.equal(B.view(torch.int8), ref[1].view(torch.int8))):
+                        raise RuntimeError(f"setting {cfg} changed the results of {bench}")
                 results.append((timed(), cfg))
         best_ms, best = min(results, key=lambda r: r[0])
         if best_ms >= base_ms:

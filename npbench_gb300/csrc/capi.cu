@@ -128,7 +128,7 @@ cudaError_t encode_3d(CUtensorMap* map, int esize, const void* base, const uint6
 
 extern "C" {
 
-const char* npbgb_version(void) { return "npbgb 0.1.0 sm_103a"; }
+const char* npbgb_version(void) { return "npbgb 0.2.0 sm_103a"; }
 
 const char* npbgb_last_error(void) { return npbgb::g_last_error; }
 
