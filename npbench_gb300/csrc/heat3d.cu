@@ -394,6 +394,17 @@ int32_t launch_ldg(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tstep
   return cuda_status(e, "heat3d_ldg");
 }
 
+// Binary32 arrays beyond the L2 whose rows strips of 32 columns (TMA) cut with less waste
+// than strips of 30 (heat_rows.cu): there the columns loaded in vain cost bandwidth.
+// TMA's time over the rows', arrays of 120 MB and more: n2 = 64 (90 columns for 64) 0.88 to
+// 0.90, 96 (120 for 96) 0.93, 128 (150 for 128) 0.94 to 0.96, 160 (180 for 160) 0.98, 192
+// (210 for 192) 0.99, 256 (270 for 256) 0.99 to 1.03, 80 (90 for 96) 1.03; of 100 MB 0.95,
+// 1.02, 0.99, 1.04 and 1.01; of 80 MB and less 1.1 to 1.5.
+bool tma_strips_pay(int64_t n0, int64_t n1, int64_t n2) {
+  const int64_t rows = 30 * cdiv(n2 - 2, 30), tma = 32 * cdiv(n2 - 2, 32);  // columns loaded
+  return n0 * n1 * n2 * 8 > (10 * rows > 13 * tma ? 95000000 : 110000000) && 25 * rows > 27 * tma;
+}
+
 template <typename T, bool FX>
 int32_t run_single(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tsteps, cudaStream_t st) {
   if (tsteps <= 1 || n0 < 3 || n1 < 3 || n2 < 3) return NPBGB_OK;
@@ -407,12 +418,12 @@ int32_t run_single(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tstep
       if (r != NPBGB_ERR_STATE) return r;
     }
   }
-  // binary32 streams rows with plain loads (heat_rows.cu) unless a setting of the TMA
-  // form is made and TMA can copy the arrays: faster at every size measured (ms,
-  // rows / TMA / staged: 64^3, TSTEPS=50, 0.26 / 0.38 / -; 224^3, 21, 0.64 / 0.72; 310 x
-  // 311 x 319, 11, 0.98 / - / 3.44) but 512^3 (5: 1.59 / 1.55).
+  // binary32 streams rows with plain loads (heat_rows.cu) unless TMA can copy the arrays
+  // and a setting of its form is made or that is the faster one: rows take 0.26 ms against
+  // 0.38 at 64^3, TSTEPS=50, 0.64 / 0.72 at 224^3, 21, 0.82 / 0.87 at 288^3, 11 (0.98
+  // against 3.44 staged through shared memory at 310 x 311 x 319, 11); see tma_strips_pay.
   if constexpr (sizeof(T) == 4) {
-    if (!g_cfg_heat_tma || (g_cfg_heat_rows == 0 && g_cfg_heat_stages == 0)) {
+    if (!g_cfg_heat_tma || (g_cfg_heat_rows == 0 && g_cfg_heat_stages == 0 && !tma_strips_pay(n0, n1, n2))) {
       const int32_t r = heat3d_rows_run(a, b, n0, n1, n2, tsteps, st);
       if (r != NPBGB_ERR_STATE) return r;
     }
