@@ -51,7 +51,9 @@ extern "C" {
                                      identical either way. */
 #define NPBGB_CFG_HEAT_CHUNK 2    /* axis-0 planes per CTA in heat3d; 0 = automatic */
 #define NPBGB_CFG_HEAT_TMA 3      /* 1 (default): heat3d stages planes with TMA when the
-                                     arrays allow it; 0: plain loads only */
+                                     arrays allow it, in the forms that do; 0: plain
+                                     loads only (binary32 then streams rows or, with
+                                     NPBGB_CFG_HEAT_ROWS set, stages planes) */
 #define NPBGB_CFG_JACOBI_CHUNK 4  /* rows per warp in jacobi2d; 0 = automatic */
 #define NPBGB_CFG_HEAT_ROWS 5     /* axis-1 tile rows per thread in heat3d (TMA): 1, 2, 4;
                                      0 (default) = 4 for binary32, 2 for binary64 */

@@ -423,7 +423,7 @@ int32_t run_single(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tstep
   // 0.38 at 64^3, TSTEPS=50, 0.64 / 0.72 at 224^3, 21, 0.82 / 0.87 at 288^3, 11 (0.98
   // against 3.44 staged through shared memory at 310 x 311 x 319, 11); see tma_strips_pay.
   if constexpr (sizeof(T) == 4) {
-    if (!g_cfg_heat_tma || (g_cfg_heat_rows == 0 && g_cfg_heat_stages == 0 && !tma_strips_pay(n0, n1, n2))) {
+    if (g_cfg_heat_rows == 0 && (!g_cfg_heat_tma || (g_cfg_heat_stages == 0 && !tma_strips_pay(n0, n1, n2)))) {
       const int32_t r = heat3d_rows_run(a, b, n0, n1, n2, tsteps, st);
       if (r != NPBGB_ERR_STATE) return r;
     }
@@ -457,8 +457,10 @@ int32_t run_single(T* a, T* b, int64_t n0, int64_t n1, int64_t n2, int32_t tstep
     if (r != NPBGB_ERR_STATE) return r;
   }
   if constexpr (sizeof(T) == 4) {
-    const int32_t r = heat3d_rows_run(a, b, n0, n1, n2, tsteps, st);
-    if (r != NPBGB_ERR_STATE) return r;
+    if (g_cfg_heat_tma) {
+      const int32_t r = heat3d_rows_run(a, b, n0, n1, n2, tsteps, st);
+      if (r != NPBGB_ERR_STATE) return r;
+    }
   }
   return launch_ldg<T, FX>(a, b, n0, n1, n2, tsteps, st);
 }
