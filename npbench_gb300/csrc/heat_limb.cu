@@ -82,12 +82,8 @@ __device__ __forceinline__ L3 axis(const fxl::Consts& K, const L3& c, const L3& 
   return s;
 }
 
-// The point at q whose sum has the exponent field e; out of line, rarely taken.  All
-// inputs of a sum of nothing were in limbs: it is +0 (evaluated in hardware, a field of
-// zeros took 9.0 ms at 256^3, TSTEPS=11, instead of 2.3).  Any other is evaluated in
-// hardware binary64.
-__device__ __noinline__ double other_point(const double* q, int64_t s0, int64_t s1, uint32_t e) {
-  if (e == 0u) return 0.0;
+// The point at q in hardware binary64; out of line, rarely taken.
+__device__ __noinline__ double hardware_point(const double* q, int64_t s0, int64_t s1) {
   return hcore::heat_point<double>(q[0], q[s0], q[-s0], q[s1], q[-s1], q[1], q[-1]);
 }
 
@@ -304,8 +300,12 @@ __device__ __forceinline__ int run_chunk(const double* __restrict__ src, double*
           fxl::to_f64<62>(fxl::second(q.h), fxl::second(q.m), fxl::second(q.l), fxl::second(e), K.scale));
       if (!(fxl::within<-4, 3>(fxl::first(e)) && fxl::within<-4, 3>(fxl::second(e)))) {
         const double* g = src + (o - dst);
-        if (out_a[r] && !fxl::within<-4, 3>(fxl::first(e))) va = other_point(g + off_a[r] / 8, s0, n2, fxl::first(e));
-        if (out_b[r] && !fxl::within<-4, 3>(fxl::second(e))) vb = other_point(g + off_b[r] / 8, s0, n2, fxl::second(e));
+        // All inputs of a sum of nothing (e = 0) were in limbs: it is +0.  Evaluated in
+        // hardware, a field of zeros took 9.0 ms at 256^3, TSTEPS=11, instead of 2.0.
+        if (!fxl::within<-4, 3>(fxl::first(e)))
+          va = out_a[r] && fxl::first(e) != 0u ? hardware_point(g + off_a[r] / 8, s0, n2) : 0.0;
+        if (!fxl::within<-4, 3>(fxl::second(e)))
+          vb = out_b[r] && fxl::second(e) != 0u ? hardware_point(g + off_b[r] / 8, s0, n2) : 0.0;
       }
       if (out_a[r]) *reinterpret_cast<double*>(reinterpret_cast<char*>(o) + off_a[r]) = va;
       if (out_b[r]) *reinterpret_cast<double*>(reinterpret_cast<char*>(o) + off_b[r]) = vb;
