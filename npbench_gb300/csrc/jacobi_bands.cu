@@ -886,8 +886,11 @@ cudaError_t scratch_pool(cudaMemPool_t* out) {
 //     but every pair with a value out of the limbs' range is mended out of line, and
 //     fields come to hold such values (NPBench's own initial field 0.63 against 0.35, a
 //     hot wall in a cold box 0.51 against 0.33, standard normal values 0.64 against 0.39);
-//   * binary32 of more than 2049 columns (8 a thread) with 2 pairs a thread: 300 x
-//     2990, TSTEPS=50 0.461 against 0.447 ms (700 x 2900 0.481 against 0.586);
+//   * binary32 of more than 2049 columns (8 a thread) and fewer rows than 0.29 of them,
+//     where a half-sweep gains too little on the load and the way back.  TSTEPS=16 and 40,
+//     us, chained and bands: 2300 columns, 600 rows 161, 172 and 380, 367; 750 rows 179,
+//     172 and 427, 356; 3300, 750 187, 215 and 442, 454; 900 227, 226 and 553, 479; 4096, 900
+//     226, 254 and 544, 546; 1200 265, 273 and 644, 566;
 //   * next to a tile queue, whose worker would keep the bands' CTAs waiting;
 //   * short runs, as launch, load and way back cost about 25 us and more for wide
 //     grids (binary32, TSTEPS=6 and 11: 1000^2 52 and 69 us against 55 and 91; 2500^2
@@ -898,20 +901,19 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   const bool any = g_cfg_jacobi_bands == 2;
   if (tsteps <= 1 || tsteps > (1 << 30) || ny < 4 || nx < 3 || ny > (1 << 20) || nx > 4096) return NPBGB_ERR_STATE;
   if (sizeof(T) == 8 && !(any && g_cfg_f64_emulation)) return NPBGB_ERR_STATE;
-  if (!any && queue_exists()) return NPBGB_ERR_STATE;
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
-    return NPBGB_ERR_STATE;
-  int dev = 0, smem_max = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (dev < 0 || dev >= 64) return NPBGB_ERR_STATE;
-  const size_t room = size_t(smem_max) - 1024;
   // As few columns a thread as the width allows.
   int which = 0;
   while (which < 3 && nx - 1 > int64_t(instances<T>()[which].cpt) * instances<T>()[which].compute) ++which;
   if (which == 3) return NPBGB_ERR_STATE;
   const Instance<T>& in = instances<T>()[which];
+  const bool wide = sizeof(T) == 4 && which == 2;
+  if (!any && (tsteps < (!wide ? 8 : nx > 2400 ? 20 : 16) || (wide && 100 * ny < 29 * nx))) return NPBGB_ERR_STATE;
+  if (!any && queue_exists()) return NPBGB_ERR_STATE;
+  int dev = 0, smem_max = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (dev < 0 || dev >= 64) return NPBGB_ERR_STATE;
+  const size_t room = size_t(smem_max) - 1024;
   const int compute = int(cdiv(cdiv(nx - 1, in.cpt), 32) * 32), columns = in.cpt * compute;
   // As few pairs a thread as any cluster size gives, but two (one leaves more bands
   // and their hand-offs: 150^2, binary32, TSTEPS=50 0.147 against 0.136 ms); then the
@@ -926,8 +928,9 @@ int32_t jacobi2d_bands_run(T* a, T* b, int64_t ny, int64_t nx, int32_t tsteps, c
   }
   const size_t smem = in_cluster ? in.bytes(H, compute) : 0;
   if (in_cluster == 0 || smem > room) return NPBGB_ERR_STATE;
-  const bool wide = sizeof(T) == 4 && which == 2;
-  if (!any && (tsteps < (wide ? 16 : 8) || (wide && H < 3))) return NPBGB_ERR_STATE;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
+    return NPBGB_ERR_STATE;
   const int nb = int(cdiv(interior, 2 * H)), clusters = int(cdiv(nb, in_cluster));
   const size_t mail_bytes = size_t(4) * clusters * size_t(columns) * sizeof(typename Kind<T>::Mail);
   const size_t bytes = mail_bytes + 256;  // and a counter

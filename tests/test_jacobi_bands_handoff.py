@@ -37,3 +37,30 @@ def test_bands_equal_chained_launches(dtype, shape):
         _lib.set_config(_lib.NPBGB_CFG_JACOBI_BANDS, old)
         if was:
             autotune.enable()
+
+
+# On both sides of the line for grids whose threads take eight columns.
+@pytest.mark.parametrize("shape, tsteps, one", [
+    ((600, 2300), 16, False), ((700, 2300), 16, True), ((750, 2500), 19, False), ((750, 2500), 20, True),
+    ((750, 3300), 40, False), ((1000, 3300), 20, True), ((900, 4096), 40, False), ((1200, 4096), 20, True)])
+def test_wide_grids_of_few_rows_keep_chained_launches(shape, tsteps, one):
+    import torch
+
+    from npbench_gb300 import _lib, autotune, stencils
+    A, B = (torch.rand(shape, device="cuda") for _ in range(2))
+    was = autotune.enabled()
+    autotune.disable()
+    try:
+        results = []
+        for bands in (1, 0):
+            old = _lib.set_config(_lib.NPBGB_CFG_JACOBI_BANDS, bands)
+            got, n0 = (A.clone(), B.clone()), _lib.launches()
+            stencils.jacobi_2d_kernel(tsteps, *got)
+            _lib.device_status()
+            _lib.set_config(_lib.NPBGB_CFG_JACOBI_BANDS, old)
+            results.append((got, _lib.launches() - n0))
+    finally:
+        if was:
+            autotune.enable()
+    assert results[0][1] == (1 if one else 2 * (tsteps - 1)) and results[1][1] == 2 * (tsteps - 1)
+    assert all(torch.equal(x, y) for x, y in zip(results[0][0], results[1][0]))
