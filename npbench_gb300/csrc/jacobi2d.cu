@@ -174,7 +174,8 @@ jacobi2d_limb_loop(double* a, double* b, int64_t ny, int64_t nx, int halfsweeps,
 // 56 and no neighbours to wait for at a CTA's end (1700 x 1500, TSTEPS=21: 0.530 ms
 // against 0.572; 4096^2, 5: 0.557 / 0.60; but 1000^2, 50: 0.744 / 0.711).  Rows are an
 // even number (two at a time) growing with the square root of q.  Measured best with
-// four warps at q = 0.1 to 2.2: 2 (600^2, TSTEPS=50: 0.425 ms, 4 0.532); 3.3: 4 (1403 x
+// four warps at q = 0.1 to 3.06: 2 (600^2, TSTEPS=50: 0.424 ms, 4 0.537; 650^2 0.482 and
+// 0.530; 700^2 0.512 and 0.538); 3.1: 4 (1000 x 500: 0.525, 2 0.544); 3.3: 4 (1403 x
 // 377: 0.539, 2 0.573, 6 0.652); 6.2: 6 (1000^2: 0.715, 4 0.739, 8 0.795); with one at
 // 15: 10 to 16; 30: 16 to 24; 48: 20 (2800^2, 11: 0.707, 10 0.736); 102: 24 to 32.
 struct LimbShape { int warps, chunk; };
@@ -183,7 +184,7 @@ LimbShape limb_shape(int64_t ny, int64_t nx) {
   const bool alone = q >= 9.0;
   const int64_t least = cdiv(ny - 2, 65535);  // the grid's limit
   if (g_cfg_jacobi_chunk > 0) return {alone ? 1 : kLimbWarps, int(std::max<int64_t>(g_cfg_jacobi_chunk, least))};
-  const int64_t pairs = alone ? int64_t(1.5 * std::sqrt(q) + 0.5) : std::max<int64_t>(int64_t(1.2 * std::sqrt(q) + 0.15), 1);
+  const int64_t pairs = alone ? int64_t(1.5 * std::sqrt(q) + 0.5) : q < 3.08 ? 1 : int64_t(1.2 * std::sqrt(q) + 0.15);
   return {alone ? 1 : kLimbWarps, int(std::max<int64_t>(2 * pairs, least + (least & 1)))};
 }
 
