@@ -11,29 +11,32 @@ exited 0:
 ========== ============================================== ===================
 case       what                                           kernel to capture
 ========== ============================================== ===================
-heat_f64   Heat-3D 256^3 float64, TSTEPS=3 (4 launches)   heat3d_tma, -s 2
-heat_f32   Heat-3D 256^3 float32, TSTEPS=3                heat3d_tma, -s 2
-jacobi_f64 Jacobi-2D 4096^2 float64, TSTEPS=3             jacobi2d_strip, -s 2
+heat_f64   Heat-3D 256^3 float64, TSTEPS=3 (4 launches)   heat3d_limb, -s 2
+heat_signed  the same on standard normal values           heat3d_limb, -s 2
+heat_f32   Heat-3D 256^3 float32, TSTEPS=3                heat3d_rows, -s 2
+jacobi_f64 Jacobi-2D 4096^2 float64, TSTEPS=3             jacobi2d_limb, -s 2
 jacobi_f32 Jacobi-2D 4096^2 float32, TSTEPS=3             jacobi2d_strip, -s 2
 hdiff      hdiff 256x256x160 float64, 3 calls             hdiff_tile, -s 1
 vadv       vadv 256x256x160 float64, 3 calls              vadv_columns, -s 1
-cavity     cavity_flow 101x101, nt=20, nit=50, 2 calls    cavity_bands, -s 1
-batch      256 mixed Jacobi-2D grids, 2 launches          batch_persistent, -s 1
+cavity     cavity_flow 101x101, nt=20, nit=50, 2 calls    cfd_mail, -s 1
+batch      256 mixed Jacobi-2D grids, stepped, 2 passes   batch_step, -s 20
 batch_step 256 mixed grids, stepped form, one pass        batch_step, -s 20
-jacobi_f64_1000  Jacobi-2D 1000^2 float64, TSTEPS=3       jacobi2d_strip, -s 2
-jacobi1d   Jacobi-1D N=32000 float64, TSTEPS=64           jacobi1d_block, -s 2
+jacobi_f64_1000  Jacobi-2D 1000^2 float64, TSTEPS=3       jacobi2d_limb, -s 2
+jacobi_loop  Jacobi-2D 400^2 float64, TSTEPS=21           jacobi2d_limb_loop, -c 1
+jacobi1d   Jacobi-1D N=32000 float64, TSTEPS=64           jacobi1d_block, -s 1
+jacobi1d_f32  Jacobi-1D N=32000 float32, TSTEPS=401       jacobi1d_resident, -c 1
 fdtd       FDTD-2D 1000x1200 float64, TMAX=3 (6 launches) fdtd_e / fdtd_h, -s 1
 heat_f32_tb Heat-3D 416^3 float32, TSTEPS=6: 4 two-step   heat3d_tb2, -s 1
            launches, then one single-step pair
-heat_f32_384 Heat-3D 384^3 float32, TSTEPS=3, one step    heat3d_tma, -s 2
+heat_f32_384 Heat-3D 384^3 float32, TSTEPS=3, one step    heat3d_rows, -s 2
            per launch
-heat_f32_512 Heat-3D 512^3 float32, TSTEPS=3 (automatic   heat3d_tma, -s 2
-           5-plane chunks)
+heat_f32_512 Heat-3D 512^3 float32, TSTEPS=3 (tuned:      heat3d_tma, -s 2
+           4-plane chunks)
 heat_f32_chunks  timing sweep (CUDA events, no ncu) of    -
            the binary32 Heat-3D plane chunks and forms,
            256^3 to 640^3, TSTEPS=21; one JSON line per size
-jacobi_bands_1000  Jacobi-2D 1000^2 float64, TSTEPS=10,   jacobi2d_bands, -c 1
-           one launch with the bands in shared memory
+jacobi_bands_1000  Jacobi-2D 1000^2 float64, TSTEPS=10,   (launched under
+           one launch with the bands in shared memory     ncu without clusters)
 jacobi_f64_fx  Jacobi-2D 4096^2 float64, TSTEPS=3, every  jacobi2d_strip, -s 2
            warp in fixed point
 jacobi_f64_hw  the same, every warp on hardware binary64  jacobi2d_strip, -s 2
@@ -116,6 +119,19 @@ def run(case):
         A, B = workloads.uniform_heat((256,) * 3, dt, seed=0)
         a, b = torch.from_numpy(A).to(dev), torch.from_numpy(B).to(dev)
         stencils.heat_3d_kernel(3, a, b)
+    elif case == "heat_signed":
+        gen = torch.Generator(device=dev)
+        gen.manual_seed(3)
+        a = torch.randn((256,) * 3, generator=gen, device=dev, dtype=torch.float64)
+        stencils.heat_3d_kernel(3, a, a.clone())
+    elif case == "jacobi_loop":
+        A, B = workloads.uniform_pair((400, 400), np.float64, seed=0)
+        a, b = torch.from_numpy(A).to(dev), torch.from_numpy(B).to(dev)
+        stencils.jacobi_2d_kernel(21, a, b)
+    elif case == "jacobi1d_f32":
+        A, B = workloads.init_jacobi_1d(32000, np.float32)
+        a, b = torch.from_numpy(A).to(dev), torch.from_numpy(B).to(dev)
+        stencils.jacobi_1d_kernel(401, a, b)
     elif case in ("jacobi_f64", "jacobi_f32"):
         dt = np.float64 if case.endswith("64") else np.float32
         A, B = workloads.uniform_pair((4096, 4096), dt, seed=0)
