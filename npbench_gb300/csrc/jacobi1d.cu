@@ -87,9 +87,12 @@ template <typename T>
 int32_t run(T* a, T* b, int64_t n, int32_t tsteps, cudaStream_t st) {
   if (tsteps <= 1 || n < 3) return NPBGB_OK;
   // binary32 hands values on within one launch (jacobi1d_resident.cu) unless a setting
-  // of the chained form is made; runs of a few chained launches are faster chained.
+  // of the chained form is made (the defaults are none: reading one gives the value in
+  // effect, and callers put back what they read); runs of a few chained launches are
+  // faster chained.
   if constexpr (sizeof(T) == 4) {
-    if (g_cfg_jacobi1d_ctas == 0 && g_cfg_jacobi1d_depth == 0 && tsteps >= kLeastResident) {
+    if (jacobi1d_effective_ctas() == kDefaultCtas && jacobi1d_effective_depth() == kDefaultDepth &&
+        tsteps >= kLeastResident) {
       const int32_t r = jacobi1d_resident_run(a, b, n, tsteps, st);
       if (r != NPBGB_ERR_STATE) return r;
     }

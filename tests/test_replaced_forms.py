@@ -70,6 +70,21 @@ def test_binary32_jacobi_1d_launches(n, tsteps, one):
     assert (_lib.launches() - n0 == 1) == one
 
 
+def test_settings_put_back_leave_the_default_form(settings):
+    import torch
+
+    from npbench_gb300 import stencils
+    A, B = (torch.rand(32000, device="cuda") for _ in range(2))
+    for key, other in ((_lib.NPBGB_CFG_JACOBI1D_CTAS, 2), (_lib.NPBGB_CFG_JACOBI1D_DEPTH, 16)):
+        old = _lib.get_config(key)
+        for value, one in ((other, False), (old, True)):
+            settings(key, value)
+            n0 = _lib.launches()
+            stencils.jacobi_1d_kernel(100, A, B)
+            _lib.device_status()
+            assert (_lib.launches() - n0 == 1) == one
+
+
 def _round_up(n):
     return -(-n // 256) * 256
 
